@@ -248,11 +248,12 @@ void DecodePlan::refresh() {
 }
 
 // Rows of the [parts, rows] buffers that carry the per-row partial sums of squares between two kernels: the largest count
-// any producer of a residual stream of width D may write - one partial per feature tile of the streaming kernel (whose
-// tiles shrink to 8 features when the inner size is large, so up to D / 8), of the dense kernels (D / 128) or of the
-// cross-GPU sum - whatever the row count of the pass (the producers choose their tiling from the inner sizes D and F).
+// any producer of a residual stream of width D may write - one partial per feature tile of the streaming kernel (D / 16), of the
+// dense kernels (D / 128) or of the cross-GPU sum, whatever the row count of the pass; never below D / 8, which callers may have
+// laid their own buffers out for.
 Index shadow_partial_rows(Index D, Index F) {
-    Index parts = 1;
+    if (D <= 0 || F <= 0) return 0;
+    Index parts = (D + 7) / 8;
     for (const Index rows : {Index{1}, Index{kShadowDenseRows}})
         for (const Index inner : {D, F})
             parts = std::max<Index>(parts, b200_linear_shadow_parts(rows, inner, D));

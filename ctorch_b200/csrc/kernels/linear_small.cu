@@ -345,7 +345,7 @@ extern "C" int32_t b200_linear_shadow_parts(int64_t rows, int64_t in, int64_t ou
 extern "C" const char* b200_linear_shadow_kernel(int64_t rows, int64_t in, int64_t out) {
     // mirrors the dispatch of launch_linear_stream / launch_linear_gemm for a shadow call with bf16 weights
     if (rows <= 0 || in <= 0 || out <= 0 || rows > INT32_MAX) return "";
-    if (rows >= b200::kGemmRows || in > 2048) {
+    if (!b200::linear_stream_takes(static_cast<int>(rows), static_cast<int>(in))) {
         if (rows >= b200::kGemmRows && out <= 64 && rows <= 512) return "linear_thin_kernel";
         return b200::linear_decode_takes(static_cast<int>(rows)) ? "linear_decode_kernel" : "linear_gemm_kernel";
     }

@@ -1,21 +1,10 @@
-// Streaming skinny linear for bf16 weights and up to 16 activation rows per tile (the decode batch):
-// y = epilogue(rmsnorm?(x) @ W^T).  The work is weight streaming, so the kernel is built around keeping many
-// kilobytes of weights in flight per SM:
-//   * persistent CTAs (one per SM) walk feature tiles of TF rows of W; a producer warp streams every tile through
-//     a ring of shared-memory slots with bulk TMA copies (cp.async.bulk, one per weight row, mbarrier completion,
-//     no multicast, no descriptor to fetch) and runs ahead across tile boundaries; the first slots are requested
-//     before the activations are touched, so DRAM latency overlaps the prologue; rows land with a padded stride
-//     so that ldmatrix reads them without bank conflicts;
-//   * the activation rows are staged once per CTA: RMSNorm in f64 (src/kernels/cpu/normalization.cpp:39-51 of the
-//     reference), then split into bf16 hi + bf16 lo so that the tensor cores see ~16 mantissa bits of the f32 value;
-//   * eight consumer warps split K: warp w takes the 16-column k-steps w, w+8, ... of every stage, multiplies the
-//     [16 x 16] activation fragments (hi and lo) with the [16 x TF] weight fragments using mma.sync m16n8k16 bf16
-//     with f32 accumulation (fragments via ldmatrix from the swizzled stage), and the per-warp partial sums are
-//     added through shared memory before the shared epilogue (linear_common.cuh) runs.
-// Rows beyond 16 are covered by blockIdx.y (weights then come from L2).  Shapes it does not take (f32 weights,
-// in > 2048 or in % 8 != 0) stay on the CUDA-core kernel.
+// Skinny linears for bf16 weights and up to 16 activation rows (decode batches): y = epilogue(rmsnorm?(x) @ W^T).  Two kernels:
+//   * linear_stream_kernel: activations that arrive as two bf16 planes - every linear of a bf16 decode step;
+//   * linear_staged_kernel: f32 activation rows, normalised and split while they are staged (logits behind a prefill, plain linears).
 #include "linear_common.cuh"
+#include "mma.cuh"
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -44,26 +33,284 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t address) 
 __device__ __forceinline__ void ldmatrix_x2(uint32_t (&r)[2], uint32_t address) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(address));
 }
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void consumer_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kConsumers * 32) : "memory"); }
 
-// 1-D bulk copy global -> shared of `bytes` (multiple of 16, both addresses 16-byte aligned), completion on an mbarrier.
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+// ---- streaming kernel: activations as bf16 planes ---------------------------------------------------------------------------
+// Bound by weight streaming, so nothing stands between memory and the tensor cores: 16 bytes of a weight row are a lane's fragment of
+// mma.m16n8k16 as they lie.  Lane (g, t) of a warp fetches entries [8t, 8t + 8) of a 32-column chunk of weight rows g and g + 8, and of
+// activation row g; the products of a chunk take the columns in an order of their own (product 0: entries 8t .. 8t + 3 of every lane,
+// product 1: 8t + 4 .. 8t + 7), the same on both sides, so nothing is shuffled.  Weights are the M side (16 features), activation rows
+// the N side (8 or 16 tokens, two planes).
+//   * A group of warps (8 or 16, see few_groups) owns tiles of 16 features and shares out the chunks of K.  Every lane has a ring of its own
+//     in shared memory, filled by cp.async and read back by the same lane: no barrier, and 128 KB in flight per SM across tile borders,
+//     started before the wait for the predecessor (6.5 TB/s over 148 SMs need about 45 KB at a microsecond of latency; a ring of 80 KB
+//     in half the registers, so that two kernels share an SM, spilled and was a quarter slower).
+//   * Activations stay in registers over all tiles where a warp has at most kFewKeep chunks (in <= 2048), all requested at once.
+//   * The warps' partial sums meet in shared memory, in two buffers, so that a tile costs one barrier; the first 64 * NT threads finish
+//     it (one row, two adjacent features each) while the other warps are in the next tile.
+// Measured back to back, weights from memory, 1 | 16 rows, against a ring of whole tiles of 8 - 32 features with all activations staged first
+// and two barriers a tile: 2048 -> 16384 SwiGLU 31.5 | 22.6 -> 12.8 | 15.6 us (5.2 | 4.3 TB/s), 2048 -> 32000 argmax 54.0 | 43.9 -> 21.9 |
+// 26.1 us (6.0 TB/s), 2048 -> 3072 15.4 | 6.9 -> 5.0 | 6.1, 768 -> 768 6.6 | 3.9 -> 2.7 | 3.1, 768 -> 32000 18.3 | 14.5 -> 10.8 | 13.6.
+struct FewParams {
+    LinearParams base;
+    int tiles;   // ceil(out / 16)
+};
+constexpr int kFewFeatures = 16, kFewKeep = 4, kFewDepth = 8, kFewWarps = 16;
+
+template <int NT, int WARPS, int EPI>
+__global__ void __launch_bounds__(kFewWarps * 32, 1) linear_stream_kernel(const __grid_constant__ FewParams fp) {
+    constexpr int kPitch = 8 * NT + 1, kGroups = kFewWarps / WARPS, kSpan = WARPS * 32;   // kSpan: columns that a group takes side by side
+    const LinearParams& p = fp.base;
+    extern __shared__ __align__(16) uint4 ring[];   // [warps][kFewDepth][2][32]
+    __shared__ float partial[kGroups][2][WARPS][kFewFeatures * kPitch];
+    __shared__ float slices[kGroups][WARPS * 4 / NT][8 * NT];   // sums of squares: slices of the producer's partials x rows
+    const int groups = blockDim.x / kSpan, group = threadIdx.x / kSpan, thread = threadIdx.x % kSpan;
+    const int warp = thread >> 5, lane = thread & 31, g = lane >> 2, t = lane & 3;
+    const int first_tile = blockIdx.x * groups + group, tile_step = gridDim.x * groups;
+    const int per_tile = (p.in + kSpan - 1) / kSpan, column0 = warp * 32 + 8 * t;
+    const uint4 zeros = make_uint4(0u, 0u, 0u, 0u);
+
+    const uint4* mine = ring + (threadIdx.x >> 5) * (kFewDepth * 64) + lane;
+    const uint32_t ring_at = smem_u32(mine);
+    // the next chunk of this warp, zeros where there is none
+    int load_feature = first_tile * kFewFeatures + g, load_column = column0, load_slot = 0;
+    const auto* load_from = static_cast<const __nv_bfloat16*>(p.weight) + static_cast<int64_t>(load_feature) * p.in + column0;
+    const int64_t upper_rows = static_cast<int64_t>(8) * p.in, next_tile = static_cast<int64_t>(tile_step * kFewFeatures) * p.in - (per_tile - 1) * kSpan;
+    auto load = [&] {
+        const bool live = load_column < p.in && load_feature < p.out, upper = load_column < p.in && load_feature + 8 < p.out;
+        const uint32_t to = ring_at + load_slot * 1024;
+        copy_async_16(to, live ? load_from : p.weight, live);
+        copy_async_16(to + 512, upper ? load_from + upper_rows : p.weight, upper);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        load_slot = load_slot + 1 == kFewDepth ? 0 : load_slot + 1;
+        load_column += kSpan;
+        if (load_column - column0 < per_tile * kSpan) {
+            load_from += kSpan;
+        } else {
+            load_column = column0;
+            load_feature += tile_step * kFewFeatures;
+            load_from += next_tile;
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < kFewDepth; ++i) load();
+
+    // Weights are constants; the activations (and residual, cache, q) come from the preceding kernels.
+    grid_dependency_wait();
+    uint4 hi[kFewKeep][NT], lo[kFewKeep][NT];
+    auto load_x = [&](int step0) {   // this warp's activations of chunks step0 .. step0 + kFewKeep - 1
+#pragma unroll
+        for (int u = 0; u < kFewKeep; ++u) {
+            const int column = (step0 + u) * kSpan + column0;
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                const bool live = n * 8 + g < p.rows && column < p.in;
+                const int64_t at = static_cast<int64_t>(n * 8 + g) * p.in + column;
+                hi[u][n] = live ? *reinterpret_cast<const uint4*>(p.x_hi + at) : zeros;
+                lo[u][n] = live && p.x_lo ? *reinterpret_cast<const uint4*>(p.x_lo + at) : zeros;
+            }
+        }
+    };
+    load_x(0);
+    constexpr int kSlices = WARPS * 4 / NT;
+    if (p.sumsq_in) {   // read again behind the first tile's barrier
+        const int r = thread & (8 * NT - 1), slice = thread / (8 * NT);
+        float sum = 0.0f;
+        if (r < p.rows)
+#pragma unroll 4
+            for (int i = slice; i < p.parts_in; i += kSlices) sum += __ldg(p.sumsq_in + static_cast<int64_t>(i) * p.rows + r);
+        slices[group][slice][r] = sum;
+    }
+    grid_launch_dependents();
+
+    // this thread's share of a tile's epilogue
+    const int my_row = thread >> 3, my_pair = (thread & 7) * 2;
+    const bool finishes = thread < 64 * NT;
+    float row_scale = 1.0f;
+    bool scaled = p.sumsq_in == nullptr;
+    Candidate running{-INFINITY, INT32_MAX};
+    float carried[2] = {0.0f, 0.0f};
+    float acc[NT][4], rest[NT][4];   // sums of the hi and of the lo plane: two chains of products
+    int parity = 0, slot = 0;
+    auto finish = [&](int tile) {
+        float* mine = partial[group][parity][warp];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            mine[g * kPitch + n * 8 + 2 * t] = acc[n][0] + rest[n][0];
+            mine[g * kPitch + n * 8 + 2 * t + 1] = acc[n][1] + rest[n][1];
+            mine[(g + 8) * kPitch + n * 8 + 2 * t] = acc[n][2] + rest[n][2];
+            mine[(g + 8) * kPitch + n * 8 + 2 * t + 1] = acc[n][3] + rest[n][3];
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kSpan) : "memory");
+        if (finishes) {   // whole warps
+            if (!scaled) {
+                float sum = 0.0f;
+                for (int slice = 0; slice < kSlices; ++slice) sum += slices[group][slice][my_row];
+                row_scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, static_cast<float>(p.in)), static_cast<float>(p.eps))));
+                scaled = true;
+            }
+            float a = 0.0f, b = 0.0f;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) {
+                a += partial[group][parity][w][my_pair * kPitch + my_row];
+                b += partial[group][parity][w][(my_pair + 1) * kPitch + my_row];
+            }
+            a *= row_scale;
+            b *= row_scale;
+            const int row = my_row, feature0 = tile * kFewFeatures + my_pair;
+            const bool live = row < p.rows && feature0 < p.out, second = feature0 + 1 < p.out;
+            if constexpr (EPI == B200_EPI_RESIDUAL) {
+                if (live) {
+                    const int64_t at = static_cast<int64_t>(row) * p.out + feature0;
+                    a = __fadd_rn(carried[0], a);
+                    b = second ? __fadd_rn(carried[1], b) : 0.0f;
+                    p.y[at] = a;
+                    if (second) p.y[at + 1] = b;
+                    store_copies(p, at, a, b, second);
+                }
+                // a, b are the new residual-stream values: shadow for the consumer, row sums of squares for its norm
+                float square = live ? a * a + b * b : 0.0f;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) square += __shfl_xor_sync(0xffffffffu, square, o);
+                if (p.sumsq_out && my_pair == 0 && row < p.rows) p.sumsq_out[static_cast<int64_t>(tile) * p.rows + row] = square;
+                if (p.out_hi && live) {   // out is even here
+                    float wa = 1.0f, wb = 1.0f;
+                    if (p.out_norm_weight) {
+                        if (p.out_norm_dtype == B200_BF16) {
+                            const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(p.out_norm_weight) + feature0;
+                            wa = __bfloat162float(w[0]);
+                            wb = __bfloat162float(w[1]);
+                        } else {
+                            const float* w = static_cast<const float*>(p.out_norm_weight) + feature0;
+                            wa = w[0];
+                            wb = w[1];
+                        }
+                    }
+                    const float va = out_norm_value(p, a, wa, p.out_norm_bias ? p.out_norm_bias[feature0] : 0.0f);
+                    const float vb = out_norm_value(p, b, wb, p.out_norm_bias ? p.out_norm_bias[feature0 + 1] : 0.0f);
+                    uint32_t h, l;
+                    pack_planes(va, vb, h, l);
+                    const int64_t at = static_cast<int64_t>(row) * p.out + feature0;
+                    *reinterpret_cast<uint32_t*>(p.out_hi + at) = h;
+                    *reinterpret_cast<uint32_t*>(p.out_lo + at) = l;
+                }
+            } else if constexpr (EPI == B200_EPI_ARGMAX) {
+                if (live) {
+                    const Candidate best = pair_candidate(feature0, a, b, p.out);
+                    if (preferred(best, running)) running = best;
+                }
+            } else if (live) {
+                linear_epilogue<EPI>(p, row, feature0, a, b);
+                if constexpr (EPI == B200_EPI_SWIGLU) {
+                    if (p.out_hi) {
+                        const __nv_bfloat16 h = __float2bfloat16_rn(a);
+                        const int64_t at = row * p.out_stride + (feature0 >> 1);
+                        p.out_hi[at] = h;
+                        p.out_lo[at] = __float2bfloat16_rn(a - __bfloat162float(h));
+                    }
+                }
+            }
+        }
+        parity ^= 1;   // (a warp reaches this buffer again only past the next tile's barrier, which the readers pass afterwards)
+    };
+    for (int tile = first_tile; tile < fp.tiles; tile += tile_step) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[n][i] = rest[n][i] = 0.0f;
+        if constexpr (EPI == B200_EPI_RESIDUAL) {   // the values that the epilogue adds, requested under the products
+            const int feature0 = tile * kFewFeatures + my_pair;
+            if (finishes && my_row < p.rows && feature0 < p.out) {
+                const float* from = p.residual + static_cast<int64_t>(my_row) * p.out + feature0;
+                carried[0] = from[0];
+                carried[1] = feature0 + 1 < p.out ? from[1] : 0.0f;
+            }
+        }
+        for (int step0 = 0; step0 < per_tile; step0 += kFewKeep) {
+            if (per_tile > kFewKeep && (step0 > 0 || tile != first_tile)) load_x(step0);
+#pragma unroll
+            for (int u = 0; u < kFewKeep; ++u) {
+                if (step0 + u >= per_tile) break;
+                asm volatile("cp.async.wait_group %0;" ::"n"(kFewDepth - 1) : "memory");
+                const uint4 w0 = mine[slot * 64], w1 = mine[slot * 64 + 32];
+                const uint32_t first[4] = {w0.x, w1.x, w0.y, w1.y}, second[4] = {w0.z, w1.z, w0.w, w1.w};
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    mma_16816(acc[n], first, hi[u][n].x, hi[u][n].y);
+                    mma_16816(rest[n], first, lo[u][n].x, lo[u][n].y);
+                    mma_16816(acc[n], second, hi[u][n].z, hi[u][n].w);
+                    mma_16816(rest[n], second, lo[u][n].z, lo[u][n].w);
+                }
+                slot = slot + 1 == kFewDepth ? 0 : slot + 1;
+                load();   // into the slot that was just read
+            }
+        }
+        finish(tile);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if constexpr (EPI == B200_EPI_ARGMAX) {   // one candidate per row and group
+        if (finishes) {
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const Candidate other{__shfl_xor_sync(0xffffffffu, running.value, o), __shfl_xor_sync(0xffffffffu, running.index, o)};
+                if (preferred(other, running)) running = other;
+            }
+            if (my_pair == 0 && my_row < p.rows) {
+                p.best_value[static_cast<int64_t>(first_tile) * p.rows + my_row] = running.value;
+                p.best_index[static_cast<int64_t>(first_tile) * p.rows + my_row] = running.index;
+            }
+        }
+    }
 }
 
+// How a launch is cut.  Up to 1024 columns, eight warps hold their activations in registers as well as sixteen do, and two groups of eight
+// cover each other's barriers and epilogues (768 -> 32000, one row: 14.3 us with one group of sixteen, 10.8 with two of eight); a second
+// group only where there is more than a tile per SM.
+struct FewGroups {
+    int warps, per_cta, ctas;
+    int total() const { return per_cta * ctas; }
+};
+FewGroups few_groups(int in, int out, int sms) {
+    const int tiles = (out + kFewFeatures - 1) / kFewFeatures, warps = in <= kFewKeep * 8 * 32 ? 8 : kFewWarps;
+    const int per_cta = warps == 8 && tiles > sms ? 2 : 1;
+    return {warps, per_cta, std::min((tiles + per_cta - 1) / per_cta, sms)};
+}
+
+// Rows up to which inner sizes beyond 2048 take the streaming kernel too.  There a group fetches its activations again for every tile (4 bytes
+// a value and row for every 32 bytes of weights).  1 | 4 rows, here against linear_decode_kernel: 8192 -> 2048 9.9 | 10.2 us against
+// 12.1 | 12.5, 4096 -> 28672 39.0 | 40.5 against 41.9 | 42.1; with 8 rows the activations are a fifth of the traffic and the lead is gone.
+constexpr int kFewWideRows = 4;
+
+template <int NT, int WARPS> int launch_few(const FewParams& fp, int epilogue, const FewGroups& cut, cudaStream_t stream) {
+    auto go = [&](auto kernel) {
+        const int threads = cut.per_cta * WARPS * 32;
+        B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewDepth * kFewWarps * 1024));
+        return cuda_status(launch_dependent(kernel, dim3(cut.ctas), dim3(threads), threads * kFewDepth * 32, stream, fp), "linear_stream_kernel launch");
+    };
+    switch (epilogue) {
+    case B200_EPI_STORE: return go(linear_stream_kernel<NT, WARPS, B200_EPI_STORE>);
+    case B200_EPI_RESIDUAL: return go(linear_stream_kernel<NT, WARPS, B200_EPI_RESIDUAL>);
+    case B200_EPI_SWIGLU: return go(linear_stream_kernel<NT, WARPS, B200_EPI_SWIGLU>);
+    case B200_EPI_QKV: return go(linear_stream_kernel<NT, WARPS, B200_EPI_QKV>);
+    case B200_EPI_ARGMAX: return go(linear_stream_kernel<NT, WARPS, B200_EPI_ARGMAX>);
+    }
+    return B200_UNSUPPORTED;
+}
+
+// ---- staged kernel: f32 activation rows -----------------------------------------------------------------------------------
+// Persistent CTAs (one per SM) walk feature tiles of TF rows of W; a producer warp streams every tile through a ring of shared-memory
+// slots with bulk TMA copies (one per weight row, mbarrier completion, no multicast) and runs ahead across tile boundaries.  The
+// activation rows are staged once per CTA: RMSNorm (src/kernels/cpu/normalization.cpp:39-51 of the reference), then split into bf16
+// hi + lo.  Eight consumer warps split K, fragments via ldmatrix (padded rows: no bank conflicts), and add their partial sums through
+// shared memory before the shared epilogue.  Rows beyond 16 are covered by blockIdx.y (weights then come from L2).
+// Shapes it does not take (f32 weights, in > 2048 or in % 8 != 0) stay on the CUDA-core kernel.
 // Shared memory map (offsets from a 128-byte aligned base):
 //   [0, slots * slot_bytes)         weight tiles, [TF rows][in_padded + 8] bf16 each (row stride = 16 mod 128 bytes)
 //   then x_hi, x_lo                 [16][in_padded + 8] bf16 each
 //   then partial sums               [8 warps][16 rows][TF] f32
 //   then mbarriers                  full[slots], empty[slots]
-template <int TF, int EPI, bool SHADOW>
-__global__ void __launch_bounds__(kThreads, 2) linear_stream_kernel(const StreamParams sp) {
+template <int TF, int EPI>
+__global__ void __launch_bounds__(kThreads, 2) linear_staged_kernel(const StreamParams sp) {
     constexpr int NT = TF / 8;  // n-tiles of 8 features
     const LinearParams& p = sp.base;
     extern __shared__ uint8_t smem_raw[];
@@ -76,9 +323,6 @@ __global__ void __launch_bounds__(kThreads, 2) linear_stream_kernel(const Stream
     float* partial = reinterpret_cast<float*>(x_lo + kRows * x_stride);
     uint64_t* full = reinterpret_cast<uint64_t*>(partial + kConsumers * kRows * TF);
     uint64_t* empty = full + sp.slots;
-    uint64_t* xbar = empty + sp.slots;                                   // shadow input copies
-    float* row_scale = reinterpret_cast<float*>(xbar + 1);               // [16]
-    float* slices = row_scale + kRows;                                   // [16 slices][16 rows] sums of squares
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row0 = blockIdx.y * kRows;
@@ -93,7 +337,6 @@ __global__ void __launch_bounds__(kThreads, 2) linear_stream_kernel(const Stream
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], kConsumers);
         }
-        mbar_init(xbar, 1);
         consumers_gave_up = 0;
         mbar_fence_init();
     }
@@ -137,71 +380,6 @@ __global__ void __launch_bounds__(kThreads, 2) linear_stream_kernel(const Stream
 
     // Weights are constants; the activations (and residual, cache, q) come from the preceding kernels.
     grid_dependency_wait();
-    if constexpr (SHADOW) {
-        // ---- consumers, shadow input: the rows arrive by bulk copy in their final form (one memory round trip, no
-        // instructions); the row scales come from the producer's per-tile sums of squares.
-        const int valid = p.rows - row0 < kRows ? p.rows - row0 : kRows;
-        if (warp == 0) {
-            if (lane == 0) mbar_expect_tx(xbar, static_cast<uint32_t>(2 * valid * p.in * 2));
-            __syncwarp();
-            const int r = lane & 15;
-            if (r < valid) {
-                const __nv_bfloat16* plane = lane < 16 ? p.x_hi : p.x_lo;
-                bulk_load((lane < 16 ? x_hi : x_lo) + r * x_stride, plane + static_cast<int64_t>(row0 + r) * p.in,
-                          static_cast<uint32_t>(p.in * 2), xbar);
-            }
-        }
-        // Row scales: 16 threads per row-partial slice read the producer's per-tile sums of squares with independent
-        // loads, the slices are added in a fixed order (deterministic), thread r finishes row r.
-        {
-            const int r = threadIdx.x & 15, slice = threadIdx.x >> 4;  // 16 slices of the partials
-            float mine = 0.0f;
-            if (p.sumsq_in && row0 + r < p.rows) {
-                float v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int i = slice + u * 16;
-                    v[u] = i < p.parts_in ? __ldg(p.sumsq_in + static_cast<int64_t>(i) * p.rows + row0 + r) : 0.0f;
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) mine += v[u];
-                for (int i = slice + 128; i < p.parts_in; i += 16) mine += __ldg(p.sumsq_in + static_cast<int64_t>(i) * p.rows + row0 + r);
-            }
-            slices[slice * kRows + r] = mine;
-        }
-        // The pad columns (in .. in_padded + 8) of all rows and the rows beyond the batch are zeros.
-        {
-            const int pad_words = (x_stride - p.in) >> 1;
-            for (int i = threadIdx.x; i < 2 * kRows * pad_words; i += kConsumers * 32) {
-                const int line = i / pad_words, word = i - line * pad_words;  // line = plane * 16 + row
-                reinterpret_cast<uint32_t*>((line >= kRows ? x_lo : x_hi) + (line & (kRows - 1)) * x_stride + p.in)[word] = 0u;
-            }
-            const int row_words = p.in >> 1;
-            for (int i = threadIdx.x; i < 2 * (kRows - valid) * row_words; i += kConsumers * 32) {
-                const int line = i / row_words, word = i - line * row_words;
-                const int plane = line / (kRows - valid), r = valid + line - plane * (kRows - valid);
-                reinterpret_cast<uint32_t*>((plane ? x_lo : x_hi) + r * x_stride)[word] = 0u;
-            }
-        }
-        if (!mbar_wait(xbar, 0)) {
-            if (lane == 0) atomicExch(sp.status, B200_DEVICE_TIMEOUT);
-            *static_cast<volatile int*>(&consumers_gave_up) = 1;
-        }
-        consumer_barrier();
-        if (*static_cast<volatile int*>(&consumers_gave_up)) return;   // the activations never arrived: same decision in every consumer warp
-        if (threadIdx.x < kRows) {  // read again only after the barrier that follows the first tile's products
-            float scale = 1.0f;
-            if (p.sumsq_in && row0 + threadIdx.x < p.rows) {
-                float total = 0.0f;
-#pragma unroll
-                for (int slice = 0; slice < 16; ++slice) total += slices[slice * kRows + threadIdx.x];
-                scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(p.in)), static_cast<float>(p.eps))));
-            }
-            row_scale[threadIdx.x] = scale;
-        }
-        // Only now may the successor start: its weight prefetch would otherwise queue ahead of the copies above.
-        grid_launch_dependents();
-    } else
     // ---- consumers: stage the activations (the weight stream is already in flight) ----
     // Warp w owns rows w and w+8.  Both rows are read with independent 16-byte loads into registers (one L2 round
     // trip), reduced to their RMS (f32 squares per lane, f64 across lanes and for the square root), normalised,
@@ -281,25 +459,12 @@ __global__ void __launch_bounds__(kThreads, 2) linear_stream_kernel(const Stream
     const uint32_t a_hi = smem_u32(x_hi) + a_lane, a_lo = smem_u32(x_lo) + a_lane;
     const int ksteps = (p.in + 15) >> 4;
 
-    // B200_EPI_ARGMAX: the row candidates this thread has seen over the CTA's tiles (one per pass of the finishing loop)
-    Candidate running[TF > 32 ? 2 : 1];
-#pragma unroll
-    for (int i = 0; i < (TF > 32 ? 2 : 1); ++i) running[i] = Candidate{-INFINITY, INT32_MAX};
-
     bool alive = true;
     for (int t = 0; t < my_tiles && alive; ++t) {
         const int tile = blockIdx.x + t * gridDim.x;
         float acc[NT][4];
 #pragma unroll
         for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
-        // The residual values this thread will add in the tile's epilogue are requested now, under the products.
-        float2 carried = make_float2(0.0f, 0.0f);
-        if constexpr (SHADOW && EPI == B200_EPI_RESIDUAL && TF <= 32) {
-            const int r = threadIdx.x / (TF / 2), f = (threadIdx.x - r * (TF / 2)) * 2;
-            const int row = row0 + r, feature0 = tile * TF + f;
-            if (r < kRows && row < p.rows && feature0 + 1 < p.out)
-                carried = *reinterpret_cast<const float2*>(p.residual + static_cast<int64_t>(row) * p.out + feature0);
-        }
         {
             const int s = t % sp.slots;
             const uint32_t phase = (t / sp.slots) & 1;
@@ -320,17 +485,17 @@ __global__ void __launch_bounds__(kThreads, 2) linear_stream_kernel(const Stream
                 if constexpr (NT == 1) {
                     uint32_t b[2];
                     ldmatrix_x2(b, b_lane + column_bytes);
-                    mma_bf16(acc[0], ah, b[0], b[1]);
-                    mma_bf16(acc[0], al, b[0], b[1]);
+                    mma_16816(acc[0], ah, b[0], b[1]);
+                    mma_16816(acc[0], al, b[0], b[1]);
                 } else {
 #pragma unroll
                     for (int n = 0; n < NT; n += 2) {
                         uint32_t b[4];
                         ldmatrix_x4(b, b_lane + static_cast<uint32_t>(n * 8 * x_stride * 2) + column_bytes);
-                        mma_bf16(acc[n], ah, b[0], b[1]);
-                        mma_bf16(acc[n], al, b[0], b[1]);
-                        mma_bf16(acc[n + 1], ah, b[2], b[3]);
-                        mma_bf16(acc[n + 1], al, b[2], b[3]);
+                        mma_16816(acc[n], ah, b[0], b[1]);
+                        mma_16816(acc[n], al, b[0], b[1]);
+                        mma_16816(acc[n + 1], ah, b[2], b[3]);
+                        mma_16816(acc[n + 1], al, b[2], b[3]);
                     }
                 }
             }
@@ -366,92 +531,16 @@ __global__ void __launch_bounds__(kThreads, 2) linear_stream_kernel(const Stream
             }
             const int row = row0 + r, feature0 = tile * TF + f;
             const bool live = in_tile && row < p.rows && feature0 < p.out;
-            if constexpr (SHADOW) {
-                if (in_tile) { a *= row_scale[r]; b *= row_scale[r]; }
-            }
-            if constexpr (SHADOW && EPI == B200_EPI_RESIDUAL && TF <= 32) {
-                if (live) {  // out is even on the shadow path, so the pair is complete
-                    a = __fadd_rn(carried.x, a);
-                    b = __fadd_rn(carried.y, b);
-                    *reinterpret_cast<float2*>(p.y + static_cast<int64_t>(row) * p.out + feature0) = make_float2(a, b);
-                    store_copies(p, static_cast<int64_t>(row) * p.out + feature0, a, b, true);
-                }
-            } else {
-                if (live) linear_epilogue<EPI>(p, row, feature0, a, b);
-            }
-            if constexpr (SHADOW && EPI == B200_EPI_RESIDUAL) {
-                // a, b now hold the new residual-stream values: shadow for the consumer, row sums of squares for its norm
-                float square = live ? a * a + (feature0 + 1 < p.out ? b * b : 0.0f) : 0.0f;
-#pragma unroll
-                for (int o = 1; o < TF / 2; o <<= 1) square += __shfl_xor_sync(0xffffffffu, square, o);
-                if (p.sumsq_out && f == 0 && in_tile && row < p.rows) p.sumsq_out[static_cast<int64_t>(tile) * p.rows + row] = square;
-                if (p.out_hi && live) {
-                    float wa = 1.0f, wb = 1.0f;
-                    if (p.out_norm_weight) {
-                        const bool second = feature0 + 1 < p.out;
-                        if (p.out_norm_dtype == B200_BF16) {
-                            const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(p.out_norm_weight) + feature0;
-                            wa = __bfloat162float(w[0]);
-                            wb = second ? __bfloat162float(w[1]) : 0.0f;
-                        } else {
-                            const float* w = static_cast<const float*>(p.out_norm_weight) + feature0;
-                            wa = w[0];
-                            wb = second ? w[1] : 0.0f;
-                        }
-                    }
-                    const float va = out_norm_value(p, a, wa, p.out_norm_bias ? p.out_norm_bias[feature0] : 0.0f);
-                    const float vb = out_norm_value(p, b, wb, p.out_norm_bias ? p.out_norm_bias[feature0 + 1] : 0.0f);
-                    const __nv_bfloat162 hi = __floats2bfloat162_rn(va, vb);
-                    const __nv_bfloat162 lo = __floats2bfloat162_rn(va - __low2float(hi), vb - __high2float(hi));
-                    const int64_t at = static_cast<int64_t>(row) * p.out + feature0;  // out is even on this path
-                    *reinterpret_cast<__nv_bfloat162*>(p.out_hi + at) = hi;
-                    *reinterpret_cast<__nv_bfloat162*>(p.out_lo + at) = lo;
-                }
-            }
-            if constexpr (EPI == B200_EPI_ARGMAX) {
-                // the TF/2 threads of a row are consecutive lanes: butterfly to the row's candidate of this tile
-                Candidate best = live ? pair_candidate(feature0, a, b, p.out) : Candidate{-INFINITY, INT32_MAX};
-#pragma unroll
-                for (int o = 1; o < TF / 2; o <<= 1) {
-                    const Candidate other{__shfl_xor_sync(0xffffffffu, best.value, o), __shfl_xor_sync(0xffffffffu, best.index, o)};
-                    if (preferred(other, best)) best = other;
-                }
-                if (preferred(best, running[base / (kConsumers * 32)])) running[base / (kConsumers * 32)] = best;
-            }
-            if constexpr (SHADOW && EPI == B200_EPI_SWIGLU) {
-                if (p.out_hi && live) {
-                    const __nv_bfloat16 hi = __float2bfloat16_rn(a);
-                    const int64_t at = row * p.out_stride + (feature0 >> 1);
-                    p.out_hi[at] = hi;
-                    p.out_lo[at] = __float2bfloat16_rn(a - __bfloat162float(hi));
-                }
-            }
+            if (live) linear_epilogue<EPI>(p, row, feature0, a, b);
         }
         consumer_barrier();
     }
-    if constexpr (EPI == B200_EPI_ARGMAX) {
-        // one candidate per row and CTA: thread (row r, first pair) holds the best of the CTA's tiles
-#pragma unroll
-        for (int base = 0; base < kRows * (TF / 2); base += kConsumers * 32) {
-            const int i = base + threadIdx.x;
-            const int r = i / (TF / 2), f = i - r * (TF / 2);
-            if (alive && f == 0 && i < kRows * (TF / 2) && row0 + r < p.rows) {
-                p.best_value[static_cast<int64_t>(blockIdx.x) * p.rows + row0 + r] = running[base / (kConsumers * 32)].value;
-                p.best_index[static_cast<int64_t>(blockIdx.x) * p.rows + row0 + r] = running[base / (kConsumers * 32)].index;
-            }
-        }
-    }
-}
-
-template <int TF, int EPI, bool SHADOW> int launch_mode(const StreamParams& sp, size_t smem, int ctas, int row_tiles, cudaStream_t stream) {
-    auto kernel = linear_stream_kernel<TF, EPI, SHADOW>;
-    B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    return cuda_status(launch_dependent(kernel, dim3(ctas, row_tiles), dim3(kThreads), smem, stream, sp), "linear_stream_kernel launch");
 }
 
 template <int TF, int EPI> int launch_tile(const StreamParams& sp, size_t smem, int ctas, int row_tiles, cudaStream_t stream) {
-    return sp.base.x_hi ? launch_mode<TF, EPI, true>(sp, smem, ctas, row_tiles, stream)
-                        : launch_mode<TF, EPI, false>(sp, smem, ctas, row_tiles, stream);
+    auto kernel = linear_staged_kernel<TF, EPI>;
+    B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    return cuda_status(launch_dependent(kernel, dim3(ctas, row_tiles), dim3(kThreads), smem, stream, sp), "linear_staged_kernel launch");
 }
 
 template <int EPI> int pick_tile(const StreamParams& sp, size_t smem, int ctas, int row_tiles, cudaStream_t stream) {
@@ -492,25 +581,19 @@ bool choose_tiling(int in, int out, int sms, StreamParams& sp, size_t& smem) {
 
 }  // namespace
 
+bool linear_stream_takes(int rows, int in) { return rows < kGemmRows && (in <= kMaxIn || rows <= kFewWideRows); }
+
 int linear_stream_parts(int rows, int in, int out) {
     if ((in & 7) || in <= 0 || out <= 0) return 0;
-    if (rows >= kGemmRows || in > kMaxIn) return linear_gemm_parts(rows, in, out);
-    int device = -1;
-    if (cudaGetDevice(&device) != cudaSuccess) { cudaGetLastError(); device = -1; }   // no device: the figures of a 148-SM part
-    StreamParams sp{};
-    size_t smem = 0;
-    return choose_tiling(in, out, sm_count(device), sp, smem) ? sp.tiles : 0;
+    return linear_stream_takes(rows, in) ? (out + kFewFeatures - 1) / kFewFeatures : linear_gemm_parts(rows, in, out);
 }
 
 int linear_argmax_parts(int rows, int in, int out) {
     if ((in & 7) || in <= 0 || out <= 0) return 0;
-    if (rows >= kGemmRows || in > kMaxIn) return linear_gemm_parts(rows, in, out);
+    if (!linear_stream_takes(rows, in)) return linear_gemm_parts(rows, in, out);
     int device = -1;
-    if (cudaGetDevice(&device) != cudaSuccess) { cudaGetLastError(); device = -1; }
-    StreamParams sp{};
-    size_t smem = 0;
-    if (!choose_tiling(in, out, sm_count(device), sp, smem)) return 0;
-    return sp.tiles < sm_count(device) ? sp.tiles : sm_count(device);   // one candidate slice per CTA
+    if (cudaGetDevice(&device) != cudaSuccess) { cudaGetLastError(); device = -1; }   // no device: the figures of a 148-SM part
+    return few_groups(in, out, sm_count(device)).total();   // one candidate slice per group
 }
 
 // ---- thin outputs (adapter down-projections: a few dozen output features) for passes the dense kernel would serve ----
@@ -580,14 +663,22 @@ int launch_linear_stream(const LinearParams& p, int epilogue, cudaStream_t strea
         && p.weight_dtype == B200_BF16 && (p.in & 7) == 0
         && ((reinterpret_cast<uintptr_t>(p.weight) | reinterpret_cast<uintptr_t>(p.x_hi) | reinterpret_cast<uintptr_t>(p.x_lo)) & 15) == 0)
         return launch_linear_thin(p, stream);
-    if (p.x_hi && (p.rows >= kGemmRows || p.in > kMaxIn)) return launch_linear_gemm(p, epilogue, stream);
-    if (p.x_hi && !p.x_lo) return B200_UNSUPPORTED;   // the streaming kernel always multiplies both planes
-    if (p.weight_dtype != B200_BF16 || p.in > kMaxIn || (p.in & 7) || (reinterpret_cast<uintptr_t>(p.weight) & 15))
+    if (p.x_hi) {
+        if (!linear_stream_takes(p.rows, p.in)) return launch_linear_gemm(p, epilogue, stream);
+        if (p.weight_dtype != B200_BF16 || (p.in & 7) || (p.out_hi && (p.out & 1))
+            || ((reinterpret_cast<uintptr_t>(p.weight) | reinterpret_cast<uintptr_t>(p.x_hi) | reinterpret_cast<uintptr_t>(p.x_lo)) & 15))
+            return B200_UNSUPPORTED;
+        if (!p.x_lo && p.in <= kMaxIn) return B200_UNSUPPORTED;   // one plane: a form of the tensor-core kernels only
+        int device = 0;
+        B200_CUDA(cudaGetDevice(&device));
+        const FewParams fp{p, (p.out + kFewFeatures - 1) / kFewFeatures};
+        const FewGroups cut = few_groups(p.in, p.out, sm_count(device));
+        if (p.rows <= 8) return cut.warps == 8 ? launch_few<1, 8>(fp, epilogue, cut, stream) : launch_few<1, 16>(fp, epilogue, cut, stream);
+        return cut.warps == 8 ? launch_few<2, 8>(fp, epilogue, cut, stream) : launch_few<2, 16>(fp, epilogue, cut, stream);
+    }
+    if (p.weight_dtype != B200_BF16 || p.in > kMaxIn || (p.in & 7) || (reinterpret_cast<uintptr_t>(p.weight) & 15)
+        || (reinterpret_cast<uintptr_t>(p.x) & 15))
         return B200_UNSUPPORTED;
-    if (p.x_hi ? ((reinterpret_cast<uintptr_t>(p.x_hi) | reinterpret_cast<uintptr_t>(p.x_lo)) & 15) || !p.x_lo
-               : (reinterpret_cast<uintptr_t>(p.x) & 15) != 0)
-        return B200_UNSUPPORTED;
-    if (p.out_hi && (p.out & 1)) return B200_UNSUPPORTED;
     int device = 0;
     B200_CUDA(cudaGetDevice(&device));
     const int sms = sm_count(device);
@@ -606,7 +697,6 @@ int launch_linear_stream(const LinearParams& p, int epilogue, cudaStream_t strea
     case B200_EPI_RESIDUAL: return pick_tile<B200_EPI_RESIDUAL>(sp, smem, ctas, row_tiles, stream);
     case B200_EPI_SWIGLU: return pick_tile<B200_EPI_SWIGLU>(sp, smem, ctas, row_tiles, stream);
     case B200_EPI_QKV: return pick_tile<B200_EPI_QKV>(sp, smem, ctas, row_tiles, stream);
-    case B200_EPI_ARGMAX: return p.x_hi ? pick_tile<B200_EPI_ARGMAX>(sp, smem, ctas, row_tiles, stream) : B200_UNSUPPORTED;
     }
     return B200_UNSUPPORTED;
 }

@@ -353,6 +353,53 @@ def test_shadow_protocol_norm_linear_residual(rows, inner, out):
     assert rel(osq.cpu().numpy().sum(axis=0), (want.astype(np.float64) ** 2).sum(axis=1)) < 1e-4
 
 
+@pytest.mark.parametrize("rows,inner,out", [(1, 8, 2), (1, 2048, 3072), (4, 14336, 4096), (3, 4104, 1001), (8, 2040, 16), (9, 1032, 2369 * 2), (16, 768, 32000), (13, 40, 130)])
+def test_streaming_linear_at_the_edges_of_its_tiles(rows, inner, out):
+    """Shadow linears of at most 16 rows: 8 | 9 rows (one or two token tiles), chunks of 32 columns and tiles of 16 features that end early, fewer
+    chunks than warps, less and more than a tile per CTA; store, residual and SwiGLU results and the greedy choice.  The planes hold 16 bits
+    of the activations exactly, so what is left are f32 sums of `inner` terms: 2e-5 as for the other shadow linears."""
+    l = B.lib()
+    g = torch.Generator(device="cuda").manual_seed(rows + inner + out)
+    x = torch.randn((rows, inner), generator=g, device="cuda")
+    hi = x.bfloat16()
+    lo = (x - hi.float()).bfloat16()
+    w = (torch.randn((out, inner), generator=g, device="cuda") * inner ** -0.5).bfloat16()
+    squares = torch.rand((5, rows), generator=g, device="cuda") * inner
+    scale = (squares.double().sum(0) / inner + 1e-5).rsqrt()[:, None]
+    want = ((hi.double() + lo.double()) @ w.double().T) * scale
+    residual = torch.randn((rows, out), generator=g, device="cuda")
+    parts = l.b200_linear_shadow_parts(rows, inner, out)
+    candidates = l.b200_linear_argmax_parts(rows, inner, out)
+    assert l.b200_linear_shadow_kernel(rows, inner, out) == b"linear_stream_kernel" and parts > 0 and candidates > 0
+
+    def call(epilogue, **more):
+        args = B.ShadowLinearArgs(x_hi=hi.data_ptr(), x_lo=lo.data_ptr(), rows=rows, inner=inner, weight=w.data_ptr(), out=out,
+                                  sumsq_in=squares.data_ptr(), parts_in=5, eps=1e-5, epilogue=epilogue, **more)
+        B.kcheck(l.b200_linear_shadow(C.byref(args), stream()))
+        torch.cuda.synchronize()
+
+    def close(got, expected):
+        return float((got.double() - expected).norm() / expected.norm()) < 2e-5
+    torch.cuda.synchronize()
+    y = torch.full((rows, out), float("nan"), device="cuda")
+    call(0, y=y.data_ptr())
+    assert close(y, want)
+    y.fill_(float("nan"))
+    partial = torch.full((parts, rows), float("nan"), device="cuda")
+    call(1, y=y.data_ptr(), residual=residual.data_ptr(), sumsq_out=partial.data_ptr())
+    assert close(y, want + residual.double()) and close(partial.sum(0), (want + residual.double()).square().sum(1))
+    if out % 2 == 0:
+        planes = [torch.full((rows, out // 2), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+        call(2, out_hi=planes[0].data_ptr(), out_lo=planes[1].data_ptr())
+        assert close(planes[0].double() + planes[1].double(), torch.nn.functional.silu(want[:, ::2]) * want[:, 1::2])
+    value = torch.full((candidates, rows), float("nan"), device="cuda")
+    index = torch.full((candidates, rows), -1, dtype=torch.int32, device="cuda")
+    call(4, best_value=value.data_ptr(), best_index=index.data_ptr())
+    call(0, y=y.data_ptr())
+    assert torch.equal(value.max(0).values, y.max(1).values)
+    assert torch.equal(index.gather(0, value.argmax(0)[None])[0].long(), y.argmax(1))
+
+
 def test_shadow_protocol_swiglu_and_attention_output():
     l = B.lib()
     rng = np.random.default_rng(77)
