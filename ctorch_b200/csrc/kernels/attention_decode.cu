@@ -125,9 +125,13 @@ __device__ __forceinline__ int balanced_pages_per_split(int pages, int planned) 
     return needed > 0 ? (pages + needed - 1) / needed : planned;
 }
 
+constexpr int kMostClustered = 8;   // CTAs of a cluster, the largest portable size
+
 // MULTI: items of several positions (prefill chunks); the decode instantiation keeps one position per item and one key
 // count for all of its rows.
-template <int HD, int STAGES, bool MULTI>
+// CLUSTERED: the splits of an item (grid y) are a thread-block cluster that merges them through distributed shared memory; every CTA
+// stays to the end, with pages or without.
+template <int HD, int STAGES, bool MULTI, bool CLUSTERED>
 __global__ void __launch_bounds__(kFastThreads) attention_mma_kernel(const __grid_constant__ CUtensorMap kmap,
                                                                      const __grid_constant__ CUtensorMap vmap,
                                                                      const AttnParams p) {
@@ -153,10 +157,11 @@ __global__ void __launch_bounds__(kFastThreads) attention_mma_kernel(const __gri
     const int base_len = p.kv.lengths[sequence];
     const int kv_len = base_len + (p.causal ? t_first + t_count : 0);   // keys the item's last position sees
     int page_end = (kv_len + kFastPageSize - 1) / kFastPageSize;
-    const int per_split = balanced_pages_per_split(page_end, p.pages_per_split);
+    const int per_split = CLUSTERED ? (page_end + static_cast<int>(gridDim.y) - 1) / static_cast<int>(gridDim.y)
+                                    : balanced_pages_per_split(page_end, p.pages_per_split);
     const int page_begin = split * per_split;
     if (page_end > page_begin + per_split) page_end = page_begin + per_split;
-    if (page_begin >= page_end) return;  // uniform for the CTA
+    if (!CLUSTERED && page_begin >= page_end) return;  // uniform for the CTA
     const int pages = page_end - page_begin;
     const int group = p.heads / p.kv.kv_heads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -310,6 +315,9 @@ __global__ void __launch_bounds__(kFastThreads) attention_mma_kernel(const __gri
 
     float* merge_o = reinterpret_cast<float*>(smem);                       // [warps][group][HD]
     float* merge_ml = merge_o + kConsumerWarps * 16 * HD;                   // [warps][16][2]
+    float* split_o = merge_ml + kConsumerWarps * 16 * 2;                    // CLUSTERED: what the CTA adds to the item, [group][HD], and
+    float* split_ml = split_o + 16 * HD;                                    //   [group][2] (max, sum)
+    static_assert((kConsumerWarps + 1) * 16 * (HD + 2) * 4 <= S::stages * S::stage_bytes);
     if (warp < kConsumerWarps) {
         const int g = lane >> 2, t = lane & 3;
 #pragma unroll
@@ -343,6 +351,11 @@ __global__ void __launch_bounds__(kFastThreads) attention_mma_kernel(const __gri
             acc += weight * merge_o[(w * 16 + r) * HD + d];
             l += weight * merge_ml[(w * 16 + r) * 2 + 1];
         }
+        if constexpr (CLUSTERED) {
+            split_o[i] = acc;
+            if (d == 0) { split_ml[2 * r] = m; split_ml[2 * r + 1] = l; }
+            continue;
+        }
         const int position = MULTI ? r / group : 0;
         const int64_t head_item = static_cast<int64_t>(row + position) * p.heads + kvh * group + (r - position * group);
         if (p.num_splits == 1) {
@@ -354,6 +367,32 @@ __global__ void __launch_bounds__(kFastThreads) attention_mma_kernel(const __gri
                 p.part_ml[(head_item * p.num_splits + split) * 2 + 1] = l;
             }
         }
+    }
+    if constexpr (CLUSTERED) {
+        cluster_sync_all();   // every split's sums are in its CTA's shared memory; each CTA finishes a share of the item
+        const uint32_t o_at = smem_u32(split_o), ml_at = smem_u32(split_ml);
+        for (int i = split * kFastThreads + threadIdx.x; i < group * HD; i += gridDim.y * kFastThreads) {
+            const int r = i / HD, d = i - r * HD;
+            float value[kMostClustered], m = -INFINITY, acc = 0.0f, l = 0.0f;
+            float2 ml[kMostClustered];
+#pragma unroll
+            for (int c = 0; c < kMostClustered; ++c) {
+                const bool there = c < static_cast<int>(gridDim.y);
+                const uint32_t pair = map_peer_shared(ml_at + r * 8, there ? c : 0), at = map_peer_shared(o_at + i * 4, there ? c : 0);
+                ml[c] = there ? make_float2(load_cluster_float(pair), load_cluster_float(pair + 4)) : make_float2(-INFINITY, 0.0f);
+                value[c] = there ? load_cluster_float(at) : 0.0f;
+            }
+#pragma unroll
+            for (int c = 0; c < kMostClustered; ++c) m = fmaxf(m, ml[c].x);
+#pragma unroll
+            for (int c = 0; c < kMostClustered; ++c) {
+                const float weight = ml[c].x == -INFINITY ? 0.0f : expf(ml[c].x - m);
+                acc += weight * value[c];
+                l += weight * ml[c].y;
+            }
+            store_result(p, (static_cast<int64_t>(row) * p.heads + kvh * group + r) * HD + d, acc / l);
+        }
+        cluster_sync_all();   // nobody leaves while a peer reads its shared memory
     }
 }
 
@@ -610,13 +649,15 @@ __global__ void __launch_bounds__(kFastThreads) attention_persistent_kernel(cons
     }
 }
 
-// Generic path: one (row, head) per CTA, four warps stride over the tokens of the split.
-constexpr int kGenericThreads = 128;
+// Generic path: one (row, head) per CTA, eight warps that take kGenericTokens tokens of the split at a time.  Bound by latency (the f32 byte
+// decoder at context 64: 8 CTAs), so the loads and the reductions of a batch of tokens are independent of each other and only one
+// softmax update follows a batch; with four warps and a token at a time the launch took 13.5 us there, now 5.4.
+constexpr int kGenericThreads = 256, kGenericWarps = kGenericThreads / 32, kGenericTokens = 8;
 constexpr int kMaxDimsPerLane = 8;  // head_dim <= 256
 
 __global__ void __launch_bounds__(kGenericThreads) attention_generic_kernel(const AttnParams p) {
-    __shared__ float merge_ml[4][2];
-    extern __shared__ float merge_o[];  // [4][head_dim]
+    __shared__ float merge_ml[kGenericWarps][2];
+    extern __shared__ float merge_o[];  // [warps][head_dim]
     grid_dependency_wait();
     grid_launch_dependents();
     const int hd = p.kv.head_dim;
@@ -640,22 +681,46 @@ __global__ void __launch_bounds__(kGenericThreads) attention_generic_kernel(cons
         acc[i] = 0.0f;
     }
     float m = -INFINITY, l = 0.0f;
-    for (int token = begin + warp; token < end; token += 4) {
-        const int64_t at = kv_offset(p.kv, sequence, token, kvh);
-        float dot = 0.0f;
+    for (int first = begin + warp * kGenericTokens; first < end; first += kGenericWarps * kGenericTokens) {
+        int64_t at[kGenericTokens];
+        float score[kGenericTokens];
 #pragma unroll
-        for (int i = 0; i < kMaxDimsPerLane; ++i) {
-            const int d = lane + 32 * i;
-            if (d < hd) dot = fmaf(qv[i], kv_load(p.kv, 0, at + d), dot);
+        for (int u = 0; u < kGenericTokens; ++u) {   // tokens past the end repeat the last one and get no weight
+            at[u] = kv_offset(p.kv, sequence, min(first + u, end - 1), kvh);
+            score[u] = 0.0f;
         }
-        const float score = warp_sum(dot) * p.scale;
-        const float m_new = fmaxf(m, score);
-        const float corr = expf(m - m_new), weight = expf(score - m_new);
-        l = l * corr + weight;
 #pragma unroll
         for (int i = 0; i < kMaxDimsPerLane; ++i) {
             const int d = lane + 32 * i;
-            if (d < hd) acc[i] = fmaf(weight, kv_load(p.kv, 1, at + d), acc[i] * corr);
+            if (d >= hd) break;
+#pragma unroll
+            for (int u = 0; u < kGenericTokens; ++u) score[u] = fmaf(qv[i], kv_load(p.kv, 0, at[u] + d), score[u]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < kGenericTokens; ++u) score[u] += __shfl_xor_sync(0xffffffffu, score[u], o);
+        float m_new = m;
+#pragma unroll
+        for (int u = 0; u < kGenericTokens; ++u) {
+            score[u] = first + u < end ? score[u] * p.scale : -INFINITY;
+            m_new = fmaxf(m_new, score[u]);
+        }
+        const float corr = expf(m - m_new);
+        l *= corr;
+#pragma unroll
+        for (int u = 0; u < kGenericTokens; ++u) {
+            score[u] = first + u < end ? expf(score[u] - m_new) : 0.0f;
+            l += score[u];
+        }
+#pragma unroll
+        for (int i = 0; i < kMaxDimsPerLane; ++i) {
+            const int d = lane + 32 * i;
+            if (d >= hd) break;
+            acc[i] *= corr;
+#pragma unroll
+            for (int u = 0; u < kGenericTokens; ++u)
+                acc[i] = first + u < end ? fmaf(score[u], kv_load(p.kv, 1, at[u] + d), acc[i]) : acc[i];
         }
         m = m_new;
     }
@@ -669,9 +734,11 @@ __global__ void __launch_bounds__(kGenericThreads) attention_generic_kernel(cons
     const int64_t head_item = static_cast<int64_t>(row) * p.heads + head;
     for (int d = threadIdx.x; d < hd; d += kGenericThreads) {
         float mm = -INFINITY;
-        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, merge_ml[w][0]);
+#pragma unroll
+        for (int w = 0; w < kGenericWarps; ++w) mm = fmaxf(mm, merge_ml[w][0]);
         float a = 0.0f, ll = 0.0f;
-        for (int w = 0; w < 4; ++w) {
+#pragma unroll
+        for (int w = 0; w < kGenericWarps; ++w) {
             const float weight = merge_ml[w][0] == -INFINITY ? 0.0f : expf(merge_ml[w][0] - mm);
             a += weight * merge_o[w * hd + d];
             ll += weight * merge_ml[w][1];
@@ -713,7 +780,18 @@ __global__ void attention_combine_kernel(const AttnParams p) {
     }
 }
 
-template <int HD, int STAGES> int launch_fast(const b200_kv_cache* cache, AttnParams p, cudaStream_t stream) {
+// CTAs per item (sequence, KV head) of a decode launch that merges inside a cluster; 1: none.  Few items leave SMs idle and a merge kernel costs
+// a launch, so the largest cluster that keeps all CTAs resident (two per SM at head_dim 64, whose smaller ring allows it) and gives each
+// two pages; contexts of more than 16 pages per CTA go to the split plan, whose CTAs are as many as the pages ask for.  Measured inside
+// decode steps, attention and merge kernel before -> one launch: 64 items of 9 pages 9.5 -> 6.9 us, 8 items of 24 pages 9.3 -> 6.0 us.
+int cluster_size(int64_t items, int pages, int head_dim, int sms) {
+    const int64_t slots = head_dim == 64 ? 2 * sms : sms;
+    for (int c = kMostClustered; c > 1; c >>= 1)
+        if (items * c <= slots && pages >= 2 * c) return pages <= 16 * c ? c : 1;
+    return 1;
+}
+
+template <int HD, int STAGES> int launch_fast(const b200_kv_cache* cache, AttnParams p, int clustered, cudaStream_t stream) {
     using S = FastShape<HD, STAGES>;
     const int blocks_per_sequence = (p.tokens_per_sequence + p.positions_per_item - 1) / p.positions_per_item;
     const int items = (p.rows / p.tokens_per_sequence) * blocks_per_sequence * p.kv.kv_heads;
@@ -725,7 +803,7 @@ template <int HD, int STAGES> int launch_fast(const b200_kv_cache* cache, AttnPa
     const int persist_bytes = S::smem_bytes + merge_bytes;   // the merge area follows the control block
     // With split items the units are dealt out in turn, which only balances when the sequences are equally long (what
     // the cache's owner knows on the host); ragged split batches keep one CTA per unit and the hardware's scheduling.
-    if (p.positions_per_item == 1 && persist_bytes <= 232448 && static_cast<int64_t>(items) * p.num_splits > sm_count(device)
+    if (clustered <= 1 && p.positions_per_item == 1 && persist_bytes <= 232448 && static_cast<int64_t>(items) * p.num_splits > sm_count(device)
         && (p.num_splits == 1 || cache->even_lengths)) {
         auto kernel = attention_persistent_kernel<HD, STAGES>;
         B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, persist_bytes));
@@ -745,7 +823,15 @@ template <int HD, int STAGES> int launch_fast(const b200_kv_cache* cache, AttnPa
         return cuda_status(launch_dependent(kernel, dim3(static_cast<unsigned>(resident)), dim3(kFastThreads), static_cast<size_t>(persist_bytes),
                                             stream, *kv_tensor_map(cache, 0), *kv_tensor_map(cache, 1), p), "attention_mma_kernel launch");
     }
-    auto kernel = p.positions_per_item > 1 ? attention_mma_kernel<HD, STAGES, true> : attention_mma_kernel<HD, STAGES, false>;
+    if (clustered > 1) {
+        auto kernel = attention_mma_kernel<HD, STAGES, false, true>;
+        B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::smem_bytes));
+        const unsigned splits = static_cast<unsigned>(clustered);
+        return cuda_status(launch_dependent_cluster(kernel, dim3(static_cast<unsigned>(items), splits), dim3(kFastThreads), S::smem_bytes, stream,
+                                                    dim3(1, splits, 1), *kv_tensor_map(cache, 0), *kv_tensor_map(cache, 1), p),
+                           "attention_mma_kernel launch");
+    }
+    auto kernel = p.positions_per_item > 1 ? attention_mma_kernel<HD, STAGES, true, false> : attention_mma_kernel<HD, STAGES, false, false>;
     B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::smem_bytes));
     const dim3 grid(static_cast<unsigned>(items), p.num_splits);
     return cuda_status(launch_dependent(kernel, grid, dim3(kFastThreads), S::smem_bytes, stream, *kv_tensor_map(cache, 0),
@@ -799,6 +885,10 @@ int attention_launch(const float* q, int64_t rows, int32_t tokens_per_sequence, 
         set_error("b200_attention_decode: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
         return B200_BAD_ARGUMENT;
     }
+    int device = 0;
+    B200_CUDA(cudaGetDevice(&device));
+    const int clustered = fast && tokens_per_sequence == 1 ? cluster_size(rows * cache->kv_heads, plan.pages_total, cache->head_dim, sm_count(device)) : 1;
+    if (clustered > 1) plan.num_splits = 1;   // merged inside the kernel: no partials in the scratch
     AttnParams p{};
     p.q = q; p.rows = static_cast<int>(rows); p.tokens_per_sequence = tokens_per_sequence; p.heads = heads; p.causal = causal;
     p.positions_per_item = positions;
@@ -815,16 +905,14 @@ int attention_launch(const float* q, int64_t rows, int32_t tokens_per_sequence, 
     if (fast) {
         // head_dim 64 with more CTAs than SMs: a 96 KB ring lets two CTAs share an SM, so one CTA's pipeline ramp and
         // drain overlap the other's streaming; with fewer CTAs each keeps the deeper ring to itself.
-        int device = 0;
-        B200_CUDA(cudaGetDevice(&device));
-        const int64_t ctas = (static_cast<int64_t>(p.rows) / tokens_per_sequence) * ((tokens_per_sequence + positions - 1) / positions)
+        const int64_t ctas = clustered * (static_cast<int64_t>(p.rows) / tokens_per_sequence) * ((tokens_per_sequence + positions - 1) / positions)
                              * p.kv.kv_heads * p.num_splits;
-        if (cache->head_dim == 128) status = launch_fast<128, 6>(cache, p, s);
-        else if (ctas > sm_count(device)) status = launch_fast<64, 6>(cache, p, s);
-        else status = launch_fast<64, 8>(cache, p, s);
+        if (cache->head_dim == 128) status = launch_fast<128, 6>(cache, p, clustered, s);
+        else if (ctas > sm_count(device)) status = launch_fast<64, 6>(cache, p, clustered, s);
+        else status = launch_fast<64, 8>(cache, p, clustered, s);
     } else {
         const dim3 grid(static_cast<unsigned>(rows) * heads, plan.num_splits);
-        status = cuda_status(launch_dependent(attention_generic_kernel, grid, dim3(kGenericThreads), sizeof(float) * 4 * cache->head_dim, s, p),
+        status = cuda_status(launch_dependent(attention_generic_kernel, grid, dim3(kGenericThreads), sizeof(float) * kGenericWarps * cache->head_dim, s, p),
                              "attention_generic_kernel launch");
     }
     if (status != B200_OK || plan.num_splits == 1) return status;

@@ -208,6 +208,12 @@ __device__ __forceinline__ float2 load_cluster_float2(uint32_t cluster_address) 
     return value;
 }
 
+__device__ __forceinline__ float load_cluster_float(uint32_t cluster_address) {
+    float value;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(value) : "r"(cluster_address));
+    return value;
+}
+
 // Number of SMs of a device (cached; 148 when the device cannot be queried).
 inline int sm_count(int device) {
     static std::mutex mutex;

@@ -259,6 +259,20 @@ def test_decode_attention_ragged(cache_dtype, hd, heads, kv_heads, lengths):
         assert rel(got[s].reshape(heads, hd), want[0, :, 0, :]) < tol, (s, length)
 
 
+@pytest.mark.parametrize("cache_dtype,hd,heads,kv_heads,lengths", [
+    (B.BF16, 64, 8, 2, [1024, 64, 1, 513]),            # clusters of eight, some of whose CTAs have no page
+    (B.BF16, 128, 16, 1, [8192, 65]),                  # eight CTAs of 16 pages
+    (B.BF16, 128, 16, 1, [8193, 4000]),                # one page more: the split plan and its merge kernel
+    (B.BF16, 64, 12, 4, [100 + 37 * s for s in range(16)]),   # four per item
+    (B.F32, 256, 4, 2, [7, 8, 9, 63, 64, 65]),         # generic path: batches of eight tokens that end early
+    (B.F32, 40, 3, 1, [1, 129]),
+    (B.BF16, 64, 20, 1, [70, 2000]),                   # 20 heads on one cached head: generic path on a bf16 pool, split
+])
+def test_decode_attention_of_few_items(cache_dtype, hd, heads, kv_heads, lengths):
+    """Launches with fewer items than SMs: splits merged inside a cluster, and the generic kernel's batches of tokens."""
+    test_decode_attention_ragged(cache_dtype, hd, heads, kv_heads, lengths)
+
+
 @pytest.mark.parametrize("cache_dtype,hd", [(B.F32, 32), (B.BF16, 64)])
 def test_chunk_attention_is_causal(cache_dtype, hd):
     """L new tokens per sequence appended to a prefix: row l sees keys 0 .. prefix + l."""
