@@ -137,6 +137,50 @@ __device__ __forceinline__ void fetch_residual_quads(const LinearParams& p, int 
     }
 }
 
+// Adapter deltas of four adjacent features of two rows: what lora_pair_delta gives for their pairs, products added in the same order, but 16
+// ranks' operands are requested together (pair by pair and eight ranks at a time the epilogue was a chain of round trips: q|k|v of the 8B
+// shape with rank 16 at 32 rows 44 us, now 28).  Not inlined: inside the epilogue it took registers from the passes without
+// adapters (168 instead of 154 in linear_decode_kernel; 2048 -> 16384 at 256 rows 36.7 us with it inlined, 32.1 so).
+struct QuadPair { float4 first, second; };
+static __device__ __noinline__ QuadPair lora_quad_deltas(const __nv_bfloat16* up, const float* low0, const float* low1, int rank) {
+    float d[2][4] = {};
+#pragma unroll 1
+    for (int j0 = 0; j0 < rank; j0 += 16) {
+        uint4 w[2][4];
+        float4 l[2][2][2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {   // (a rank that ends after eight repeats them and leaves the second half out below)
+            const int j = j0 + 8 * h < rank ? j0 + 8 * h : j0;
+#pragma unroll
+            for (int f = 0; f < 4; ++f) w[h][f] = __ldg(reinterpret_cast<const uint4*>(up + f * rank + j));
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                l[h][0][i] = __ldg(reinterpret_cast<const float4*>(low0 + j) + i);
+                l[h][1][i] = __ldg(reinterpret_cast<const float4*>(low1 + j) + i);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (j0 + 8 * h >= rank) break;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float4 a = l[h][r][0], b = l[h][r][1];
+                const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int f = 0; f < 4; ++f) {
+                    const uint32_t pairs[4] = {w[h][f].x, w[h][f].y, w[h][f].z, w[h][f].w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        d[r][f] = __fadd_rn(d[r][f], __fmul_rn(x[2 * i], bf16_lo(pairs[i])));
+                        d[r][f] = __fadd_rn(d[r][f], __fmul_rn(x[2 * i + 1], bf16_hi(pairs[i])));
+                    }
+                }
+            }
+        }
+    }
+    return {make_float4(d[0][0], d[0][1], d[0][2], d[0][3]), make_float4(d[1][0], d[1][1], d[1][2], d[1][3])};
+}
+
 // Vector form of finish_rows_pairs below: a lane holds four adjacent features, so a 128-feature row is one instruction
 // per access.  A batch of kBatch rows is worked in three straight-line phases - fetch (accumulators, residual values),
 // arithmetic, stores - with no branch between the rows, so that the rows' dependent chains (shared-memory load, scale,
@@ -416,7 +460,25 @@ __device__ __forceinline__ void finish_rows_quads(const LinearParams& p, const f
                     result[r][pass] = make_float4(v.x * scale[r], v.y * scale[r], v.z * scale[r], v.w * scale[r]);
                 }
             }
-            if (p.lora_rank > 0) {
+            if (p.lora_rank > 0 && p.weight_dtype == B200_BF16 && (p.lora_rank & 7) == 0) {
+                auto add = [&](float4& t, const float4& d) {
+                    t = make_float4(__fadd_rn(t.x, __fmul_rn(d.x, p.lora_scale)), __fadd_rn(t.y, __fmul_rn(d.y, p.lora_scale)),
+                                    __fadd_rn(t.z, __fmul_rn(d.z, p.lora_scale)), __fadd_rn(t.w, __fmul_rn(d.w, p.lora_scale)));
+                };
+#pragma unroll
+                for (int r = 0; r < kBatch; r += 2) {
+#pragma unroll
+                    for (int pass = 0; pass < kPasses; ++pass) {
+                        if (region[pass] == 1 || n0 + pass * 128 + lane * 4 >= p.out) continue;
+                        const auto* up = static_cast<const __nv_bfloat16*>(region[pass] == 0 ? p.q_up : p.v_up) + static_cast<int64_t>(local[pass]) * p.lora_rank;
+                        const float* low = p.low + (region[pass] == 2 ? p.lora_rank : 0);
+                        const QuadPair d = lora_quad_deltas(up, low + static_cast<int64_t>(m0 + rows[r]) * 2 * p.lora_rank,
+                                                            low + static_cast<int64_t>(m0 + rows[r + 1]) * 2 * p.lora_rank, p.lora_rank);
+                        add(result[r][pass], d.first);
+                        add(result[r + 1][pass], d.second);
+                    }
+                }
+            } else if (p.lora_rank > 0) {
 #pragma unroll
                 for (int r = 0; r < kBatch; ++r) {
 #pragma unroll
