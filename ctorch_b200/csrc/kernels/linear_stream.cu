@@ -609,6 +609,9 @@ __global__ void __launch_bounds__(kThinThreads) linear_thin_kernel(const LinearP
     grid_launch_dependents();
     const int row = blockIdx.x, feature0 = blockIdx.y * kThinFeatures;
     const auto* weight = static_cast<const __nv_bfloat16*>(p.weight);
+    float squares = 0.0f;   // the partial sums of the row's norm, fetched by the first warp's lanes side by side
+    if (p.sumsq_in && threadIdx.x < 32)
+        for (int i = threadIdx.x; i < p.parts_in; i += 32) squares += __ldg(p.sumsq_in + static_cast<int64_t>(i) * p.rows + row);
     float acc[kThinFeatures];
 #pragma unroll
     for (int f = 0; f < kThinFeatures; ++f) acc[f] = 0.0f;
@@ -625,8 +628,8 @@ __global__ void __launch_bounds__(kThinThreads) linear_thin_kernel(const LinearP
         }
 #pragma unroll
         for (int f = 0; f < kThinFeatures; ++f) {
-            if (feature0 + f >= p.out) break;
-            const uint4 w = __ldg(reinterpret_cast<const uint4*>(weight + static_cast<int64_t>(feature0 + f) * p.in + k));
+            // (features past the end repeat the last one: a branch here would make the eight loads a chain)
+            const uint4 w = __ldg(reinterpret_cast<const uint4*>(weight + static_cast<int64_t>(min(feature0 + f, p.out - 1)) * p.in + k));
             const uint32_t v[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[f] = fmaf(x[2 * i], bf16_lo(v[i]), fmaf(x[2 * i + 1], bf16_hi(v[i]), acc[f]));
@@ -639,16 +642,15 @@ __global__ void __launch_bounds__(kThinThreads) linear_thin_kernel(const LinearP
         for (int f = 0; f < kThinFeatures; ++f) partial[threadIdx.x >> 5][f] = acc[f];
     }
     __syncthreads();
+    if (threadIdx.x >= 32) return;
+    squares = warp_sum(squares);
     if (threadIdx.x < kThinFeatures && feature0 + threadIdx.x < p.out) {
         float total = 0.0f;
 #pragma unroll
         for (int w = 0; w < kThinThreads / 32; ++w) total += partial[w][threadIdx.x];
         float scale = 1.0f;
-        if (p.sumsq_in) {
-            float squares = 0.0f;
-            for (int i = 0; i < p.parts_in; ++i) squares += __ldg(p.sumsq_in + static_cast<int64_t>(i) * p.rows + row);
+        if (p.sumsq_in)
             scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(squares, static_cast<float>(p.in)), static_cast<float>(p.eps))));
-        }
         p.y[static_cast<int64_t>(row) * p.out + feature0 + threadIdx.x] = total * scale;
     }
 }
