@@ -96,6 +96,13 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// 2^v by the hardware unit (relative error about 2^-22; 2^-inf = 0)
+__device__ __forceinline__ float exp2_fast(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 constexpr int kConsumerWarps = 8;   // two groups of four: group g takes pages g, g+2, ... so two pages are in the
 constexpr int kGroupWarps = 4;      // tensor-core pipeline at a time; a warp owns 16 tokens of its group's page
 constexpr int kFastThreads = (kConsumerWarps + 1) * 32;
@@ -649,6 +656,181 @@ __global__ void __launch_bounds__(kFastThreads) attention_persistent_kernel(cons
     }
 }
 
+// Passes of many positions per sequence (prefill): 128 fragment rows per CTA - consecutive positions times the head group - of which each of
+// the eight warps takes 16 through all pages, so a page that is staged once serves all of them and no sums are merged in the end.
+// Products and precision are those of attention_mma_kernel (bf16 q and weights, f32 scores, softmax and sums).  Bound by the instruction
+// issue of mma.sync and the softmax around it.  Blocks of late positions, which see the most pages, come first.  8 prompts of 1024
+// positions, 32 / 8 heads of 64: attention_mma_kernel, whose CTAs take 16 rows and share out each page's tokens, 598 us (57 TFLOP/s useful),
+// this one 149 (230); 2 of 4096 positions, heads of 128: 2618 and 882 us (312 TFLOP/s).
+constexpr int kPrefillRows = kConsumerWarps * 16, kPrefillThreads = kConsumerWarps * 32;
+template <int HD> constexpr int prefill_stages() { return HD == 64 ? 5 : 4; }   // 80 KB: two CTAs per SM; 128 KB: one
+
+template <int HD>
+__global__ void __launch_bounds__(kPrefillThreads, HD == 64 ? 2 : 1) attention_prefill_kernel(const __grid_constant__ CUtensorMap kmap,
+                                                                                           const __grid_constant__ CUtensorMap vmap, const AttnParams p) {
+    using S = FastShape<HD, prefill_stages<HD>()>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::stages * S::stage_bytes);
+    uint64_t* empty = full + S::stages;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S::stages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], kConsumerWarps);
+        }
+        mbar_fence_init();
+    }
+    __syncthreads();
+    grid_dependency_wait();   // q, the cache and the lengths come from the preceding kernels
+    grid_launch_dependents();
+
+    const int group = p.heads / p.kv.kv_heads, positions = p.positions_per_item;
+    const int streams = p.kv.sequences * p.kv.kv_heads;   // (sequence, KV head)
+    const int blocks = (p.tokens_per_sequence + positions - 1) / positions;
+    const int stream = blockIdx.x % streams, block = blocks - 1 - static_cast<int>(blockIdx.x) / streams;
+    const int sequence = stream / p.kv.kv_heads, kvh = stream - sequence * p.kv.kv_heads;
+    const int t_first = block * positions, t_count = min(positions, p.tokens_per_sequence - t_first);
+    const int base_len = p.kv.lengths[sequence];
+    const int pages = (base_len + (p.causal ? t_first + t_count : 0) + kFastPageSize - 1) / kFastPageSize;
+
+    // The first lane of warp 0 requests the pages: a ring's worth here, later ones kLag pages after their stage was last read.
+    constexpr int kLag = 2;
+    const int32_t* table = p.kv.page_table + static_cast<int64_t>(sequence) * p.kv.pages_per_seq;
+    auto request = [&](int i) {
+        const int s = i % S::stages, y = (table[i] * p.kv.kv_heads + kvh) * kFastPageSize;
+        uint8_t* kdst = smem + s * S::stage_bytes;
+        uint8_t* vdst = kdst + S::tile_bytes;
+        mbar_expect_tx(&full[s], S::stage_bytes);
+#pragma unroll
+        for (int h = 0; h < S::halves; ++h) {
+            tma_load_2d(kdst + h * kHalfTileBytes, &kmap, h * 64, y, &full[s]);
+            tma_load_2d(vdst + h * kHalfTileBytes, &vmap, h * 64, y, &full[s]);
+        }
+    };
+    if (threadIdx.x == 0)
+        for (int i = 0; i < min(pages, S::stages); ++i) request(i);
+
+    // ---- this thread's two fragment rows, their activation rows and the keys each sees ----
+    const int g = lane >> 2, t = lane & 3, mi = lane >> 3, ri = lane & 7;
+    int limit[2], at_row[2], at_head[2];
+    bool live[2];
+    uint32_t qa[HD / 16][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int r = warp * 16 + g + 8 * h, position = r / group;
+        live[h] = r < group * t_count;
+        at_row[h] = sequence * p.tokens_per_sequence + t_first + position;
+        at_head[h] = kvh * group + (r - position * group);
+        limit[h] = live[h] ? base_len + (p.causal ? t_first + position + 1 : 0) : 0;
+        const float* q = p.q + (static_cast<int64_t>(at_row[h]) * p.heads + at_head[h]) * HD;
+#pragma unroll
+        for (int kk = 0; kk < HD / 16; ++kk) {
+            const int c = kk * 16 + 2 * t;
+            qa[kk][h] = live[h] ? pack_bf16(q[c], q[c + 1]) : 0u;
+            qa[kk][2 + h] = live[h] ? pack_bf16(q[c + 8], q[c + 9]) : 0u;
+        }
+    }
+    const int most = warp_max_int(max(limit[0], limit[1]));                                          // keys that some row of the warp sees
+    const int all = -warp_max_int(-min(live[0] ? limit[0] : INT32_MAX, live[1] ? limit[1] : INT32_MAX));   // keys that every live row sees
+    const float scale2 = p.scale * 1.4426950408889634f;   // scores in units of log2 e: the weights are powers of two
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
+    float o[HD / 8][4];
+#pragma unroll
+    for (int j = 0; j < HD / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
+
+    for (int i = 0; i < pages; ++i) {
+        const int s = i % S::stages;
+        if (threadIdx.x == 0 && i >= kLag && i - kLag + S::stages < pages) {
+            // (a wait that runs out leaves the page unrequested: everyone's wait for it runs out too)
+            if (mbar_wait(&empty[(i - kLag) % S::stages], ((i - kLag) / S::stages) & 1)) request(i - kLag + S::stages);
+            else atomicExch(p.status, B200_DEVICE_TIMEOUT);
+        }
+        __syncwarp();
+        if (!mbar_wait(&full[s], (i / S::stages) & 1)) {
+            if (lane == 0) atomicExch(p.status, B200_DEVICE_TIMEOUT);
+            break;
+        }
+        if (i * kFastPageSize < most) {
+            const uint32_t kbase = smem_u32(smem + s * S::stage_bytes), vbase = kbase + S::tile_bytes;
+            float sc[8][4];
+#pragma unroll
+            for (int n = 0; n < 8; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.0f;
+#pragma unroll
+            for (int kk = 0; kk < HD / 16; ++kk)
+#pragma unroll
+                for (int n = 0; n < 8; n += 2) {
+                    uint32_t r[4];
+                    ldmatrix_x4(r, kbase + tile_offset(n * 8 + (mi >> 1) * 8 + ri, 2 * kk + (mi & 1)));
+                    mma_bf16(sc[n], qa[kk], r[0], r[1]);
+                    mma_bf16(sc[n + 1], qa[kk], r[2], r[3]);
+                }
+            if ((i + 1) * kFastPageSize > all) {
+#pragma unroll
+                for (int n = 0; n < 8; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (i * kFastPageSize + n * 8 + 2 * t + (e & 1) >= limit[e >> 1]) sc[n][e] = -INFINITY;
+            }
+            float base[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float high = fmaxf(sc[0][2 * h], sc[0][2 * h + 1]);
+#pragma unroll
+                for (int n = 1; n < 8; ++n) high = fmaxf(high, fmaxf(sc[n][2 * h], sc[n][2 * h + 1]));
+                high = fmaxf(high, __shfl_xor_sync(0xffffffffu, high, 1));
+                high = fmaxf(high, __shfl_xor_sync(0xffffffffu, high, 2));
+                const float next = fmaxf(m[h], high * scale2);
+                base[h] = next == -INFINITY ? 0.0f : next;
+                const float factor = exp2_fast(m[h] - base[h]);
+                m[h] = next;
+                l[h] *= factor;
+#pragma unroll
+                for (int j = 0; j < HD / 8; ++j) { o[j][2 * h] *= factor; o[j][2 * h + 1] *= factor; }
+            }
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    sc[n][e] = exp2_fast(fmaf(sc[n][e], scale2, -base[e >> 1]));
+                    l[e >> 1] += sc[n][e];
+                }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t pa[4] = {pack_bf16(sc[2 * k][0], sc[2 * k][1]), pack_bf16(sc[2 * k][2], sc[2 * k][3]),
+                                        pack_bf16(sc[2 * k + 1][0], sc[2 * k + 1][1]), pack_bf16(sc[2 * k + 1][2], sc[2 * k + 1][3])};
+#pragma unroll
+                for (int j = 0; j < HD / 8; j += 2) {
+                    uint32_t r[4];
+                    ldmatrix_x4_trans(r, vbase + tile_offset(k * 16 + (mi & 1) * 8 + ri, j + (mi >> 1)));
+                    mma_bf16(o[j], pa, r[0], r[1]);
+                    mma_bf16(o[j + 1], pa, r[2], r[3]);
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+        if (!live[h] || limit[h] == 0) continue;   // (a row that sees no key is left as it is)
+        const int64_t at = (static_cast<int64_t>(at_row[h]) * p.heads + at_head[h]) * HD + 2 * t;
+#pragma unroll
+        for (int j = 0; j < HD / 8; ++j) {
+            const float a = o[j][2 * h] / l[h], b = o[j][2 * h + 1] / l[h];
+            if (p.out_hi) {
+                const __nv_bfloat162 hi = __floats2bfloat162_rn(a, b);
+                *reinterpret_cast<__nv_bfloat162*>(p.out_hi + at + j * 8) = hi;
+                *reinterpret_cast<__nv_bfloat162*>(p.out_lo + at + j * 8) = __floats2bfloat162_rn(a - __low2float(hi), b - __high2float(hi));
+            } else {
+                *reinterpret_cast<float2*>(p.out + at + j * 8) = make_float2(a, b);
+            }
+        }
+    }
+}
+
 // Generic path: one (row, head) per CTA, eight warps that take kGenericTokens tokens of the split at a time.  Bound by latency (the f32 byte
 // decoder at context 64: 8 CTAs), so the loads and the reductions of a batch of tokens are independent of each other and only one
 // softmax update follows a batch; with four warps and a token at a time the launch took 13.5 us there, now 5.4.
@@ -791,6 +973,25 @@ int cluster_size(int64_t items, int pages, int head_dim, int sms) {
     return 1;
 }
 
+// Whether a pass takes the prefill kernel: at least three of its eight warps have rows (below that, attention_mma_kernel's warps, which share
+// out a page's tokens, stream the cache faster), and either the context is short (a page costs a CTA here 1.0 us in a chain, there 0.4, but
+// the fixed part is 4 us against 6) or that kernel's CTAs need more than one round.  us, this | attention_mma_kernel: 1 sequence, 12 positions
+// behind 1000: 19.6 | 12.0; 32 of them: 25.6 | 44.9; 64 x 16 positions from the start: 6.0 | 26.0; heads of 128, 8 x 12 behind 500: 15.8 | 24.0.
+constexpr int kPrefillFrom = 48, kPrefillShort = 6;
+bool takes_prefill(int tokens, int group, int64_t items, int pages, int head_dim, int sms) {
+    return tokens * static_cast<int64_t>(group) >= kPrefillFrom && (pages <= kPrefillShort || items > (head_dim == 64 ? 2 : 1) * sms);
+}
+
+template <int HD> int launch_prefill(const b200_kv_cache* cache, AttnParams p, cudaStream_t stream) {
+    using S = FastShape<HD, prefill_stages<HD>()>;
+    p.positions_per_item = kPrefillRows / (p.heads / p.kv.kv_heads);
+    const int64_t ctas = static_cast<int64_t>(p.kv.sequences) * p.kv.kv_heads * ((p.tokens_per_sequence + p.positions_per_item - 1) / p.positions_per_item);
+    auto kernel = attention_prefill_kernel<HD>;
+    B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::smem_bytes));
+    return cuda_status(launch_dependent(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kPrefillThreads), S::smem_bytes, stream, *kv_tensor_map(cache, 0),
+                                        *kv_tensor_map(cache, 1), p), "attention_prefill_kernel launch");
+}
+
 template <int HD, int STAGES> int launch_fast(const b200_kv_cache* cache, AttnParams p, int clustered, cudaStream_t stream) {
     using S = FastShape<HD, STAGES>;
     const int blocks_per_sequence = (p.tokens_per_sequence + p.positions_per_item - 1) / p.positions_per_item;
@@ -907,6 +1108,10 @@ int attention_launch(const float* q, int64_t rows, int32_t tokens_per_sequence, 
         // drain overlap the other's streaming; with fewer CTAs each keeps the deeper ring to itself.
         const int64_t ctas = clustered * (static_cast<int64_t>(p.rows) / tokens_per_sequence) * ((tokens_per_sequence + positions - 1) / positions)
                              * p.kv.kv_heads * p.num_splits;
+        // pairs of results are stored together: the planes and rows that callers hand in are 4- and 8-byte aligned for that
+        const bool pairs = ((out_hi ? (reinterpret_cast<uintptr_t>(out_hi) | reinterpret_cast<uintptr_t>(out_lo)) << 1 : reinterpret_cast<uintptr_t>(out)) & 7) == 0;
+        if (tokens_per_sequence > 1 && pairs && takes_prefill(tokens_per_sequence, group, ctas, plan.pages_total, cache->head_dim, sm_count(device)))
+            return cache->head_dim == 128 ? launch_prefill<128>(cache, p, s) : launch_prefill<64>(cache, p, s);
         if (cache->head_dim == 128) status = launch_fast<128, 6>(cache, p, clustered, s);
         else if (ctas > sm_count(device)) status = launch_fast<64, 6>(cache, p, clustered, s);
         else status = launch_fast<64, 8>(cache, p, clustered, s);

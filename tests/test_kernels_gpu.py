@@ -292,6 +292,35 @@ def test_chunk_attention_is_causal(cache_dtype, hd):
     assert rel(got, want.transpose(0, 2, 1, 3)) < (1e-5 if cache_dtype == B.F32 else 1e-2)
 
 
+@pytest.mark.parametrize("hd,heads,kv_heads,n,prefix,L,causal", [
+    (64, 8, 2, 2, 0, 193, 1),      # blocks of 32 positions x 4 heads, the last one short
+    (64, 12, 4, 1, 70, 101, 1),    # a group of three: 42 positions and two rows to spare; starts inside a page
+    (128, 16, 16, 1, 5, 300, 1),   # one head per cached head: 128 positions a block
+    (128, 16, 4, 10, 640, 40, 1),  # more pages than ring stages: taken for its 400 items
+    (128, 16, 1, 2, 300, 9, 1),    # a group of 16
+    (64, 16, 1, 20, 2300, 20, 1),  # a group of 16 behind a context that the other kernels would split
+    (64, 4, 1, 1, 300, 12, 1),     # exactly the rows from which the kernel is taken
+    (64, 4, 1, 1, 500, 12, 1),     # a longer context of few items: the token-split kernel
+    (64, 8, 2, 3, 130, 33, 0),     # not causal: every row sees the prefix
+])
+def test_prefill_attention_blocks(hd, heads, kv_heads, n, prefix, L, causal):
+    """Many positions per sequence on unequal block, page and ring borders (bf16 cache; bf16 queries and weights: the tolerance of the others)."""
+    rng = np.random.default_rng(hd + heads + L)
+    cap = prefix + L
+    cache = Cache(B.BF16, n, kv_heads, hd, cap)
+    cache.set_page_table(rng.permutation(cache.pages_per_sequence() * n).astype(np.int32))
+    k, v = (rng.standard_normal((n, kv_heads, cap, hd), dtype=np.float32) for _ in range(2))
+    cache.append(k, v)
+    cache.set_lengths(np.full(n, prefix, dtype=np.int32))
+    q = rng.standard_normal((n * L, heads, hd), dtype=np.float32)
+    got = attention(q, cache, L, heads, cap, causal).reshape(n, L, heads, hd)
+    k, v = (torch.from_numpy(W.bf16_to_f32(W.bf16_bits(x))).double().repeat_interleave(heads // kv_heads, 1) for x in (k, v))
+    score = torch.from_numpy(q).double().reshape(n, L, heads, hd).transpose(1, 2) @ k.transpose(2, 3) * hd ** -0.5
+    sees = torch.arange(cap)[None] < (torch.arange(L)[:, None] + prefix + 1 if causal else prefix)
+    want = (score.masked_fill(~sees, -np.inf).softmax(-1) @ v).transpose(1, 2).numpy()
+    assert rel(got, want) < 1e-2
+
+
 def test_attention_linearity_in_values_at_long_context():
     """Size-independent property at a context the oracle would take minutes for: attention is linear in V, and
     with all keys equal it returns the mean of V."""
@@ -517,6 +546,54 @@ def test_dense_tensor_core_linear(rows, inner, out, epilogue):
         assert rel(shadow_to_f32(ohi, olo), want) < 4e-5
     if epilogue == 1:
         assert rel(osq.cpu().numpy().sum(axis=0), (want.astype(np.float64) ** 2).sum(axis=1)) < 1e-4
+
+
+@pytest.mark.parametrize("rows,inner,out,epilogue", [(1025, 72, 4704, 0),     # 171 tiles: a round of whole ones, halves behind it, the last past the end
+                                                     (1024, 520, 2080, 1),    # all tiles in halves
+                                                     (2100, 2056, 2144, 1),   # K beyond the persistent kernel's, a ragged last row tile
+                                                     (1024, 136, 4160, 2),
+                                                     (1030, 64, 5000, 0)])    # features that are no multiple of 32: not this kernel
+def test_wide_linear_tiles(rows, inner, out, epilogue):
+    """Passes of eight or more token tiles on tiles of 128 x 256: bands, halves of the last round, ragged edges."""
+    test_dense_tensor_core_linear(rows, inner, out, epilogue)
+
+
+@pytest.mark.parametrize("cache_dtype,heads,kv_heads,hd", [(B.BF16, 16, 4, 64), (B.F32, 24, 24, 32)])
+def test_wide_linear_appends_q_k_v(cache_dtype, heads, kv_heads, hd):
+    """The q|k|v epilogue of a long pass: rotation, queries, cache entries on shuffled pages, behind cached tokens."""
+    l = B.lib()
+    n, L, inner, cap = 8, 150, 256, 230
+    D, KV = heads * hd, kv_heads * hd
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    x = torch.randn((n * L, inner), generator=g, device="cuda")
+    hi = x.bfloat16()
+    lo = (x - hi.float()).bfloat16()
+    w = (torch.randn((D + 2 * KV, inner), generator=g, device="cuda") * inner ** -0.5).bfloat16()
+    cos, sin = oracle.rope_tables(hd, cap)
+    cd, sd = dev(cos), dev(sin)
+    cache = Cache(cache_dtype, n, kv_heads, hd, cap)
+    cache.set_page_table(np.random.default_rng(1).permutation(cache.pages_per_sequence() * n).astype(np.int32))
+    lengths = np.array([0, 1, 40, 63, 64, 65, 79, 80], dtype=np.int32)
+    cache.set_lengths(lengths)
+    q = torch.full((n * L, D), float("nan"), device="cuda")
+    qkv = B.QkvArgs(heads, kv_heads, hd, L, cd.data_ptr(), sd.data_ptr(), cap, cache.h.value, q.data_ptr(), 0, 0.0, None, None, None)
+    args = B.ShadowLinearArgs(x_hi=hi.data_ptr(), x_lo=lo.data_ptr(), rows=n * L, inner=inner, weight=w.data_ptr(), out=D + 2 * KV, epilogue=3, qkv=C.pointer(qkv))
+    torch.cuda.synchronize()
+    B.kcheck(l.b200_linear_shadow(C.byref(args), stream()))
+    sync()
+    y = ((hi.double() + lo.double()) @ w.double().T).cpu().numpy().reshape(n, L, -1)
+    for b in range(n):
+        at = lengths[b] + np.arange(L)
+
+        def turned(v):   # [L, heads, hd], adjacent pairs
+            u = v.reshape(L, -1, hd // 2, 2)
+            c, s = (np.asarray(t).reshape(cap, hd // 2)[at][:, None].astype(np.float64) for t in (cos, sin))
+            return np.stack([u[..., 0] * c - u[..., 1] * s, u[..., 0] * s + u[..., 1] * c], -1).reshape(v.shape)
+        assert rel(q.cpu().numpy()[b * L:(b + 1) * L], turned(y[b, :, :D].reshape(L, heads, hd)).reshape(L, D)) < 3e-5
+        tol = 3e-5 if cache_dtype == B.F32 else 5e-3
+        end = int(lengths[b]) + L
+        assert rel(cache.gather(0, end)[b][:, lengths[b]:end], turned(y[b, :, D:D + KV].reshape(L, kv_heads, hd)).transpose(1, 0, 2)) < tol
+        assert rel(cache.gather(1, end)[b][:, lengths[b]:end], y[b, :, D + KV:].reshape(L, kv_heads, hd).transpose(1, 0, 2)) < tol
 
 
 @pytest.mark.parametrize("rows,inner,vocab", [(16, 768, 32000), (5, 256, 1000), (40, 512, 5000), (32, 2048, 1024), (200, 256, 777 * 2),
