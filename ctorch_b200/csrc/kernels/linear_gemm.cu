@@ -368,6 +368,300 @@ __global__ void __launch_bounds__(kGemmThreads, 1) linear_gemm_persistent_kernel
     }
 }
 
+// ---- wide variant: long passes --------------------------------------------------------------------------------------
+// Persistent like the kernel above, with tiles of 128 tokens x 256 features: a K block then brings 64 KB into the SM for 1024 cycles of
+// products (two planes; the 128-wide tile 48 KB for 512, and an SM takes about 70 bytes a cycle from L2, which bound that kernel at 1.0 - 1.1
+// PFLOP/s issued).  Both accumulators of 256 columns fill tensor memory, the ring of three stages fills shared memory, so the epilogue
+// works from registers: a thread is one token row of the tile, 32 features at a time, every access 16 bytes (whole sectors, if not whole lines
+// per instruction; it has 17 us of products to hide under at K = 2048).  Eight warps, two per lane quarter, one for each half of the features.
+// Tiles go in bands of 16 token tiles, which stay in L2 while the weights pass by; where the last round of whole tiles would leave more than
+// half of the SMs idle, its tiles are cut in halves of 128 features.
+// us, tiles of 128 x 128 (and 128 x 256 of a CTA each beyond K = 2048) | here, 8192 rows, two planes: 2048 -> 16384 SwiGLU 969 | 697 (1.58 PFLOP/s issued), 8192 -> 2048
+// residual 467 | 384, 2048 -> 2048 residual 164 | 127, 2048 -> 3072 203 | 147, 1024 -> 8192 SwiGLU 242 | 190; 1500 rows: 221 | 159, 130 | 107, 51 | 42.
+constexpr int kWideN = 256, kWideStages = 3, kWideStageBytes = 4 * kBoxBytes, kWideBand = 16, kWideThreads = 320;
+constexpr int kWideSmem = kWideStages * kWideStageBytes + 1024 + 256;
+
+struct WidePlan { int row_tiles, feature_tiles, whole, units; };   // units: whole tiles, then halves of the tiles behind them
+
+// The tile of a unit: token tile, first feature, features (128 or 256).
+__device__ __forceinline__ void wide_place(const WidePlan& w, int unit, int out, int& m0, int& n0, int& width) {
+    const int t = unit < w.whole ? unit : w.whole + ((unit - w.whole) >> 1), half = unit < w.whole ? 0 : (unit - w.whole) & 1;
+    const int band = t / (kWideBand * w.feature_tiles), inside = t - band * kWideBand * w.feature_tiles, height = min(kWideBand, w.row_tiles - band * kWideBand);
+    const int feature_tile = inside / height;
+    m0 = (band * kWideBand + inside - feature_tile * height) * kTileM;
+    n0 = feature_tile * kWideN + half * 128;
+    width = unit >= w.whole || n0 + 128 >= out ? 128 : kWideN;
+}
+
+__device__ __forceinline__ void pack_eight(const float* v, uint4& hi, uint4& lo) {
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i] - __low2float(a), v[2 * i + 1] - __high2float(a));
+        h[i] = *reinterpret_cast<const uint32_t*>(&a);
+        l[i] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    hi = make_uint4(h[0], h[1], h[2], h[3]);
+    lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// 32 adjacent features from `feature` on of one token row; the accumulators are in tensor memory at `address`.
+template <int EPI>
+__device__ __forceinline__ void finish_chunk(const LinearParams& p, int row, int feature, uint32_t address, float scale, const int2& place, float& squares) {
+    const bool live = row < p.rows && feature < p.out;   // (out is a multiple of 32 here)
+    const int64_t at = static_cast<int64_t>(row) * p.out + feature;
+    float4 carried[8];
+    if constexpr (EPI == B200_EPI_RESIDUAL) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) carried[i] = live ? *reinterpret_cast<const float4*>(p.residual + at + 4 * i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    uint32_t r[32];
+    tmem_load_32(address, r);
+    if (!live) return;
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * scale;
+    if constexpr (EPI == B200_EPI_STORE || EPI == B200_EPI_RESIDUAL) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float4 t = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            if constexpr (EPI == B200_EPI_RESIDUAL) {
+                t = make_float4(__fadd_rn(carried[i].x, t.x), __fadd_rn(carried[i].y, t.y), __fadd_rn(carried[i].z, t.z), __fadd_rn(carried[i].w, t.w));
+                squares += t.x * t.x + t.y * t.y;
+                squares += t.z * t.z + t.w * t.w;
+                v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
+            }
+            *reinterpret_cast<float4*>(p.y + at + 4 * i) = t;
+            store_copies(p, at + 4 * i, t);
+        }
+        if constexpr (EPI == B200_EPI_RESIDUAL) {
+            if (p.out_hi) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 8) {
+                    float w[8] = {1.0f, 1.0f, 1.0f, 1.0f, 1.0f, 1.0f, 1.0f, 1.0f}, b[8] = {};
+                    if (p.out_norm_weight && p.out_norm_dtype == B200_BF16) {
+                        const uint4 q = __ldg(reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.out_norm_weight) + feature + i));
+                        const uint32_t pairs[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) { w[2 * k] = bf16_lo(pairs[k]); w[2 * k + 1] = bf16_hi(pairs[k]); }
+                    } else if (p.out_norm_weight) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) w[k] = __ldg(static_cast<const float*>(p.out_norm_weight) + feature + i + k);
+                    }
+                    if (p.out_norm_bias) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) b[k] = __ldg(p.out_norm_bias + feature + i + k);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) w[k] = out_norm_value(p, v[i + k], w[k], b[k]);
+                    uint4 hi, lo;
+                    pack_eight(w, hi, lo);
+                    *reinterpret_cast<uint4*>(p.out_hi + at + i) = hi;
+                    *reinterpret_cast<uint4*>(p.out_lo + at + i) = lo;
+                }
+            }
+        }
+    } else if constexpr (EPI == B200_EPI_SWIGLU) {
+        // (gate_j, up_j) of the interleaved weight rows; the shadow input makes this a bf16 model (see silu_fast)
+        const int j = feature >> 1;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = gated_unit(p, v[2 * i], v[2 * i + 1], true);
+        if (p.y) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4)
+                *reinterpret_cast<float4*>(p.y + static_cast<int64_t>(row) * (p.out >> 1) + j + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+        if (p.out_hi) {
+            const int64_t to = row * p.out_stride + j;
+#pragma unroll
+            for (int i = 0; i < 16; i += 8) {
+                uint4 hi, lo;
+                pack_eight(v + i, hi, lo);
+                *reinterpret_cast<uint4*>(p.out_hi + to + i) = hi;
+                *reinterpret_cast<uint4*>(p.out_lo + to + i) = lo;
+            }
+        }
+    } else {
+        // q | k | v (src/nn/decoder.cpp:77-88; src/ops/contraction.cpp:44-49; src/nn/kv_cache.cpp:24-28): the 32 features lie in one head
+        const int D = p.heads * p.head_dim, KV = p.kv_heads * p.head_dim;
+        int region = 0, local = feature;
+        if (local >= D) { region = 1; local -= D; }
+        if (region == 1 && local >= KV) { region = 2; local -= KV; }
+        const int head = local / p.head_dim, inside = local - head * p.head_dim;
+        if (region != 2 && static_cast<unsigned>(place.x) < static_cast<unsigned>(p.context)) {
+            const int64_t angle = static_cast<int64_t>(place.x) * (p.head_dim >> 1) + (inside >> 1);
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+                const float4 c4 = __ldg(reinterpret_cast<const float4*>(p.cosine + angle + i)), s4 = __ldg(reinterpret_cast<const float4*>(p.sine + angle + i));
+                const float c[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {   // adjacent-pair rotation, each product rounded before the add
+                    const float even = v[2 * (i + k)], odd = v[2 * (i + k) + 1];
+                    v[2 * (i + k)] = __fsub_rn(__fmul_rn(even, c[k]), __fmul_rn(odd, sn[k]));
+                    v[2 * (i + k) + 1] = __fadd_rn(__fmul_rn(even, sn[k]), __fmul_rn(odd, c[k]));
+                }
+            }
+        }
+        if (region == 0 || p.kv.dtype != B200_BF16) {
+            float* to = p.q_out + static_cast<int64_t>(row) * D + local;
+            if (region != 0)
+                to = static_cast<float*>(p.kv.pool[region - 1])
+                    + ((static_cast<int64_t>(place.y) * p.kv.kv_heads + head) * p.kv.page_size + place.x % p.kv.page_size) * p.kv.head_dim + inside;
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(to + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        } else {
+            auto* to = static_cast<__nv_bfloat16*>(p.kv.pool[region - 1])
+                + ((static_cast<int64_t>(place.y) * p.kv.kv_heads + head) * p.kv.page_size + place.x % p.kv.page_size) * p.kv.head_dim + inside;
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+                uint32_t h[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const __nv_bfloat162 a = __floats2bfloat162_rn(v[i + 2 * k], v[i + 2 * k + 1]);
+                    h[k] = *reinterpret_cast<const uint32_t*>(&a);
+                }
+                *reinterpret_cast<uint4*>(to + i) = make_uint4(h[0], h[1], h[2], h[3]);
+            }
+        }
+    }
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(kWideThreads, 1) linear_gemm_wide_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
+                                                                           const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GemmParams gp,
+                                                                           const WidePlan plan) {
+    constexpr uint32_t kWhole = mma_instruction_bf16(kTileM, kWideN), kHalf = mma_instruction_bf16(kTileM, 128);
+    const LinearParams& p = gp.base;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kWideStages * kWideStageBytes);
+    uint64_t* empty = full + kWideStages;
+    uint64_t* acc_full = empty + kWideStages;   // [2] the products of a tile are complete (tcgen05.commit)
+    uint64_t* acc_empty = acc_full + 2;         // [2] the epilogue has read the buffer (one arrival per epilogue warp)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k_blocks = (p.in + kBlockK - 1) / kBlockK;
+    const bool has_lo = p.x_lo != nullptr;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kWideStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 8);
+        }
+        mbar_fence_init();
+        tma_prefetch_descriptor(&map_hi);
+        tma_prefetch_descriptor(&map_lo);
+        tma_prefetch_descriptor(&map_w);
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, 2 * kWideN);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+
+    grid_dependency_wait();   // the shadow (and residual, cache, sums of squares) come from the preceding kernels
+    grid_launch_dependents();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int it = 0;   // K blocks issued so far: the ring does not restart between tiles
+            bool alive = true;
+            for (int unit = blockIdx.x; unit < plan.units && alive; unit += gridDim.x) {
+                int m0, n0, width;
+                wide_place(plan, unit, p.out, m0, n0, width);
+                const uint32_t bytes = (has_lo ? 2 * kBoxBytes : kBoxBytes) + (width == kWideN ? 2 * kBoxBytes : kBoxBytes);
+                for (int i = 0; i < k_blocks; ++i, ++it) {
+                    const int s = it % kWideStages;
+                    if (!mbar_wait(&empty[s], ((it / kWideStages) & 1) ^ 1)) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); alive = false; break; }
+                    uint8_t* stage = smem + s * kWideStageBytes;
+                    mbar_expect_tx(&full[s], bytes);
+                    tma_load_2d(stage, &map_hi, i * kBlockK, m0, &full[s]);
+                    if (has_lo) tma_load_2d(stage + kBoxBytes, &map_lo, i * kBlockK, m0, &full[s]);
+                    tma_load_2d(stage + 2 * kBoxBytes, &map_w, i * kBlockK, n0, &full[s]);
+                    if (width == kWideN) tma_load_2d(stage + 3 * kBoxBytes, &map_w, i * kBlockK, n0 + 128, &full[s]);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            int it = 0, j = 0;
+            bool alive = true;
+            for (int unit = blockIdx.x; unit < plan.units && alive; unit += gridDim.x, ++j) {
+                int m0, n0, width;
+                wide_place(plan, unit, p.out, m0, n0, width);
+                const uint32_t instruction = width == kWideN ? kWhole : kHalf, accumulator = tmem_base + static_cast<uint32_t>((j & 1) * kWideN);
+                // the epilogue of the tile that used this buffer two tiles ago must have read it (passes at once for j < 2)
+                if (!mbar_wait(&acc_empty[j & 1], ((j >> 1) & 1) ^ 1)) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); break; }
+                tc_fence_after_sync();
+                for (int i = 0; i < k_blocks; ++i, ++it) {
+                    const int s = it % kWideStages;
+                    if (!mbar_wait(&full[s], (it / kWideStages) & 1)) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); alive = false; break; }
+                    tc_fence_after_sync();
+                    const uint32_t stage = smem_u32(smem + s * kWideStageBytes);
+                    const uint64_t hi = operand_descriptor(stage), lo = operand_descriptor(stage + kBoxBytes), w = operand_descriptor(stage + 2 * kBoxBytes);
+#pragma unroll
+                    for (int k = 0; k < kBlockK / 16; ++k) {
+                        tc_mma_bf16(accumulator, hi + 2 * k, w + 2 * k, instruction, (i | k) != 0);
+                        if (has_lo) tc_mma_bf16(accumulator, lo + 2 * k, w + 2 * k, instruction, 1);
+                    }
+                    tc_commit(&empty[s]);
+                }
+                if (alive) tc_commit(&acc_full[j & 1]);
+            }
+        }
+    } else {
+        // ---- epilogue warps 2-9: TMEM lanes 32 * (warp % 4) .. + 31, features [128 * half, + 128) of the tile ----
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        int j = 0;
+        for (int unit = blockIdx.x; unit < plan.units; unit += gridDim.x, ++j) {
+            int m0, n0, width;
+            wide_place(plan, unit, p.out, m0, n0, width);
+            const int row = m0 + quarter * 32 + lane;
+            const bool mine = half * 128 < width;
+            float scale = 1.0f, squares = 0.0f;
+            int2 place = make_int2(0, 0);
+            if (mine && p.sumsq_in && row < p.rows) {
+                float total = 0.0f;
+#pragma unroll 8
+                for (int i = 0; i < p.parts_in; ++i) total += __ldg(p.sumsq_in + static_cast<int64_t>(i) * p.rows + row);
+                scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(p.in)), static_cast<float>(p.eps))));
+            }
+            if constexpr (EPI == B200_EPI_QKV) place = qkv_row_place(p, row);
+            if (!mbar_wait_relaxed(&acc_full[j & 1], (j >> 1) & 1)) {
+                if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                break;
+            }
+            tc_fence_after_sync();
+            if (mine) {
+                const uint32_t address = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>((j & 1) * kWideN + half * 128);
+#pragma unroll 1
+                for (int c = 0; c < 128; c += 32) finish_chunk<EPI>(p, row, n0 + half * 128 + c, address + c, scale, place, squares);
+                if constexpr (EPI == B200_EPI_RESIDUAL) {
+                    if (p.sumsq_out && row < p.rows && n0 + half * 128 < p.out)
+                        p.sumsq_out[static_cast<int64_t>((n0 >> 7) + half) * p.rows + row] = squares;
+                }
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[j & 1]);   // the issuing thread may reuse this accumulator
+        }
+    }
+    __syncwarp();
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, 2 * kWideN);
+    }
+}
+
 int encode_operand(CUtensorMap* map, const void* base, int rows, int columns, int box_rows) {
     encode_tiled_fn encode = tensor_map_encoder();
     if (!encode) { set_error("cuTensorMapEncodeTiled is not available from this driver"); return B200_NO_DEVICE; }
@@ -392,10 +686,30 @@ bool takes_persistent(int rows, int in, int out, int sms) {
     return row_tiles >= 8 && in <= 2048 && row_tiles * ((out + 127) / 128) > sms;
 }
 
+// Sizes that the wide kernel serves: eight or more token tiles and more 128-wide tiles than SMs, as above, at any K.
+bool takes_wide(int rows, int out, int sms) {
+    const int row_tiles = (rows + kTileM - 1) / kTileM;
+    return row_tiles >= 8 && out % 32 == 0 && static_cast<int64_t>(row_tiles) * ((out + 127) / 128) > sms;
+}
+// ... and operands: 16-byte accesses throughout, chunks of 32 features inside a head, no adapters and no greedy choice.
+bool wide_operands(const LinearParams& p, int epilogue) {
+    auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    for (int c = 0; c < p.copies; ++c)
+        if (!aligned(p.y_copy[c])) return false;
+    const bool planes = aligned(p.out_hi) && aligned(p.out_lo);
+    switch (epilogue) {
+    case B200_EPI_STORE: return aligned(p.y);
+    case B200_EPI_RESIDUAL: return aligned(p.y) && aligned(p.residual) && planes && (p.out_norm_dtype != B200_BF16 || aligned(p.out_norm_weight));
+    case B200_EPI_SWIGLU: return aligned(p.y) && planes && p.out_stride % 8 == 0;
+    case B200_EPI_QKV: return p.lora_rank == 0 && p.head_dim % 32 == 0 && aligned(p.q_out) && aligned(p.cosine) && aligned(p.sine) && aligned(p.kv.pool[0]) && aligned(p.kv.pool[1]);
+    }
+    return false;
+}
+
 int choose_tile_features(int rows, int in, int out) {
     int device = 0, sms = 148;
     if (cudaGetDevice(&device) == cudaSuccess) sms = sm_count(device);
-    if (takes_persistent(rows, in, out, sms)) return 128;
+    if (takes_persistent(rows, in, out, sms) || takes_wide(rows, out, sms)) return 128;   // (the wide kernel leaves a partial per 128 features)
     const int row_tiles = (rows + kTileM - 1) / kTileM;
     return row_tiles * ((out + 255) / 256) >= 2 * sms ? 256 : 128;
 }
@@ -473,6 +787,29 @@ int launch_persistent(int epilogue, const CUtensorMap& hi, const CUtensorMap& lo
     return B200_UNSUPPORTED;
 }
 
+int launch_wide(int epilogue, const CUtensorMap& hi, const CUtensorMap& lo, const CUtensorMap& w, const GemmParams& gp, int sms, cudaStream_t stream) {
+    WidePlan plan{};
+    plan.row_tiles = (gp.base.rows + kTileM - 1) / kTileM;
+    plan.feature_tiles = (gp.base.out + kWideN - 1) / kWideN;
+    const int64_t tiles = static_cast<int64_t>(plan.row_tiles) * plan.feature_tiles;
+    if (tiles > INT32_MAX / 2) { set_error("linear: too many tiles"); return B200_UNSUPPORTED; }
+    const int left = static_cast<int>(tiles % sms);   // tiles of the last round
+    plan.whole = static_cast<int>(2 * left <= sms ? tiles - left : tiles);
+    plan.units = plan.whole + 2 * static_cast<int>(tiles - plan.whole);
+    auto go = [&](auto kernel) {
+        B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem));
+        return cuda_status(launch_dependent(kernel, dim3(static_cast<unsigned>(plan.units < sms ? plan.units : sms)), dim3(kWideThreads), kWideSmem, stream,
+                                            hi, lo, w, gp, plan), "linear_gemm_wide_kernel launch");
+    };
+    switch (epilogue) {
+    case B200_EPI_STORE: return go(linear_gemm_wide_kernel<B200_EPI_STORE>);
+    case B200_EPI_RESIDUAL: return go(linear_gemm_wide_kernel<B200_EPI_RESIDUAL>);
+    case B200_EPI_SWIGLU: return go(linear_gemm_wide_kernel<B200_EPI_SWIGLU>);
+    case B200_EPI_QKV: return go(linear_gemm_wide_kernel<B200_EPI_QKV>);
+    }
+    return B200_UNSUPPORTED;
+}
+
 int launch_linear_gemm(const LinearParams& p, int epilogue, cudaStream_t stream) {
     if (linear_decode_takes(p.rows)) return launch_linear_decode(p, epilogue, stream);   // decode batches: weights streamed once
     if (p.weight_dtype != B200_BF16 || !p.x_hi || (p.in & 7) || (p.out_hi && (p.out & 1))
@@ -485,6 +822,12 @@ int launch_linear_gemm(const LinearParams& p, int epilogue, cudaStream_t stream)
     alignas(64) CUtensorMap hi, lo, w;
     const int sms = sm_count(device);
     const int row_tiles = (p.rows + kTileM - 1) / kTileM, tiles128 = row_tiles * ((p.out + 127) / 128);
+    if (takes_wide(p.rows, p.out, sms) && wide_operands(p, epilogue)) {
+        int status = encode_operand(&hi, p.x_hi, p.rows, p.in, kTileM);
+        if (status == B200_OK) status = encode_operand(&lo, p.x_lo ? p.x_lo : p.x_hi, p.rows, p.in, kTileM);
+        if (status == B200_OK) status = encode_operand(&w, p.weight, p.out, p.in, 128);
+        return status != B200_OK ? status : launch_wide(epilogue, hi, lo, w, gp, sms, stream);
+    }
     const bool persistent = takes_persistent(p.rows, p.in, p.out, sms);
     const int tn = persistent ? 128 : choose_tile_features(p.rows, p.in, p.out);
     int status = encode_operand(&hi, p.x_hi, p.rows, p.in, kTileM);

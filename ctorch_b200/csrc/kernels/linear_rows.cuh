@@ -139,8 +139,8 @@ __device__ __forceinline__ void fetch_residual_quads(const LinearParams& p, int 
 
 // Adapter deltas of four adjacent features of two rows: what lora_pair_delta gives for their pairs, products added in the same order, but 16
 // ranks' operands are requested together (pair by pair and eight ranks at a time the epilogue was a chain of round trips: q|k|v of the 8B
-// shape with rank 16 at 32 rows 44 us, now 28).  Not inlined: inside the epilogue it took registers from the passes without
-// adapters (168 instead of 154 in linear_decode_kernel; 2048 -> 16384 at 256 rows 36.7 us with it inlined, 32.1 so).
+// shape with rank 16 at 32 rows 44 us, now 28).  Not inlined: inside the
+// epilogue it made linear_decode_kernel spill, and linears of 64 rows without adapters took up to a quarter longer (10.0 -> 12.4 us).
 struct QuadPair { float4 first, second; };
 static __device__ __noinline__ QuadPair lora_quad_deltas(const __nv_bfloat16* up, const float* low0, const float* low1, int rank) {
     float d[2][4] = {};
