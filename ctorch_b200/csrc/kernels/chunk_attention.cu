@@ -196,12 +196,14 @@ __device__ __forceinline__ Span<V> turned_span(const ChunkParams& p, const float
     return own;
 }
 
+// Bound by its chain of loads (the row's place, its values, angles and weights), so by the CTAs that an SM holds: five, at 48 registers (8192 rows of
+// 16 / 4 heads of 64: 77 us with four at 64, 68 so; six and more spill).
 constexpr int kPrepareThreads = 256, kUnitSlice = 1024;
 // grid (rows, 1 + slices of the units)
 
 // NORM: b200_head_norm
 template <class T, int V, int NORM>
-__global__ void __launch_bounds__(kPrepareThreads) chunk_prepare_kernel(const __grid_constant__ ChunkParams p, const RowsView rows, const bool step,
+__global__ void __launch_bounds__(kPrepareThreads, 5) chunk_prepare_kernel(const __grid_constant__ ChunkParams p, const RowsView rows, const bool step,
                                                                         const __grid_constant__ Units units, const __grid_constant__ Route route) {
     extern __shared__ float logits_copy[];
     __shared__ float scratch[32];
