@@ -12,6 +12,7 @@
 //     expert_combine_kernel adds every row's results in the order of its choices: the sum does not depend on the sorting.  Where a norm
 //     stands behind the mixture it finishes the row as well (sandwich.cuh).
 #include "linear_rows.cuh"
+#include "linear_wide.cuh"
 #include "router.cuh"
 #include "rows.cuh"
 #include "sandwich.cuh"
@@ -241,7 +242,7 @@ constexpr int kGroupedThreads = 192;
 template <int SLOTS> struct GroupedShape {
     static constexpr int kPlaneBytes = SLOTS * kBlockK * 2;
     static constexpr int kStageBytes = 2 * kPlaneBytes + kWeightBytes;   // W, x_hi, x_lo of one K block
-    static constexpr int kStages = SLOTS == 128 ? 3 : SLOTS == 64 ? 5 : 8;
+    static constexpr int kStages = SLOTS == 64 ? 5 : 8;
     static constexpr int kTileBytes = SLOTS * kTileStride * 4;
     static constexpr int kTileAt = kStages * kStageBytes;
     static constexpr int kControlAt = kTileAt + kTileBytes;
@@ -520,6 +521,187 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) expert_gemm_kernel(const _
     }
 }
 
+// Tiles of 128 slots x 256 features, for slots enough to fill row tiles of 128: the ring, the two accumulators that fill tensor memory and the
+// register epilogue of linear_gemm_wide_kernel (linear_gemm.cu has the reasons), on the listed row tiles.  How many those are is known on
+// the device only, so the CTAs work out there whether the tiles of the last round are cut in halves.
+// 8192 rows, 2 of 16 experts, 2048 x 4096: up 963 -> 757 us, down 490 -> 407 (1.42 PFLOP/s issued together; 1.13 with tiles of 128 x 128).
+constexpr int kWideStages = 3, kWidePlaneBytes = kTile * kBlockK * 2, kWideStageBytes = 2 * kWidePlaneBytes + 2 * kWeightBytes;
+constexpr int kWideSmem = kWideStages * kWideStageBytes + 1024 + 256;
+
+struct WideUnits {
+    int row_tiles, feature_tiles, whole, units;
+    __device__ __forceinline__ WideUnits(int rows, int out) : row_tiles(rows), feature_tiles((out + kWideN - 1) / kWideN) {
+        const int tiles = row_tiles * feature_tiles, left = tiles % static_cast<int>(gridDim.x);
+        whole = 2 * left <= static_cast<int>(gridDim.x) ? tiles - left : tiles;
+        units = whole + 2 * (tiles - whole);
+    }
+    __device__ __forceinline__ void place(int unit, int out, int& row_tile, int& n0, int& width) const {
+        const int t = unit < whole ? unit : whole + ((unit - whole) >> 1), half = unit < whole ? 0 : (unit - whole) & 1;
+        int feature_tile;
+        tile_place(t, row_tiles, feature_tiles, row_tile, feature_tile);
+        n0 = feature_tile * kWideN + half * kTile;
+        width = unit >= whole || n0 + kTile >= out ? kTile : kWideN;
+    }
+};
+
+template <int EPI>
+__global__ void __launch_bounds__(kWideThreads, 1) expert_gemm_wide_kernel(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
+                                                                           const __grid_constant__ CUtensorMap map_w, const __grid_constant__ ExpertGemm gp) {
+    constexpr uint32_t kWhole = mma_instruction_bf16(kTile, kWideN), kHalf = mma_instruction_bf16(kTile, kTile);
+    const LinearParams& p = gp.base;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kWideStages * kWideStageBytes);
+    uint64_t* empty = full + kWideStages;
+    uint64_t* acc_full = empty + kWideStages;    // [2]
+    uint64_t* acc_empty = acc_full + 2;          // [2]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k_blocks = (p.in + kBlockK - 1) / kBlockK;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kWideStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 8);
+        }
+        mbar_fence_init();
+        tma_prefetch_descriptor(&map_hi);
+        tma_prefetch_descriptor(&map_lo);
+        tma_prefetch_descriptor(&map_w);
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, 2 * kWideN);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+
+    // a stage's barrier and weights; the bytes of the activation boxes are part of what it expects
+    auto request_weights = [&](int s, int block, int expert, int n0, int width, int boxes) {
+        uint8_t* stage = smem + s * kWideStageBytes;
+        mbar_expect_tx(&full[s], static_cast<uint32_t>((width == kWideN ? 2 : 1) * kWeightBytes + 2 * boxes * kBoxBytes));
+        tma_load_2d(stage, &map_w, block * kBlockK, expert * p.out + n0, &full[s]);
+        if (width == kWideN) tma_load_2d(stage + kWeightBytes, &map_w, block * kBlockK, expert * p.out + n0 + kTile, &full[s]);
+    };
+    int ahead = 0;   // K blocks of the first tile whose weights are on their way before the wait
+    if (gp.listed && warp == 0) {
+        const WideUnits w(*static_cast<const volatile int32_t*>(gp.tile_count), p.out);
+        if (static_cast<int>(blockIdx.x) < w.units) {
+            int row_tile, n0, width;
+            w.place(blockIdx.x, p.out, row_tile, n0, width);
+            const int4 group = *reinterpret_cast<const int4*>(gp.tiles + row_tile);
+            ahead = min(k_blocks, kWideStages);
+            if (elect_one())
+                for (int i = 0; i < ahead; ++i) request_weights(i, i, group.x, n0, width, (group.z + kBox - 1) / kBox);
+            __syncwarp();
+        }
+    }
+    grid_dependency_wait();
+    grid_launch_dependents();
+    const WideUnits w(*gp.tile_count, p.out);
+
+    if (warp == 0) {
+        int it = 0;   // K blocks issued so far: the ring does not restart between tiles
+        bool alive = true;
+        for (int unit = blockIdx.x; unit < w.units && alive; unit += gridDim.x) {
+            int row_tile, n0, width;
+            w.place(unit, p.out, row_tile, n0, width);
+            const int4 group = __ldg(gp.tiles + row_tile);
+            const int boxes = (group.z + kBox - 1) / kBox;
+            for (int i = 0; i < k_blocks; ++i, ++it) {
+                const int s = it % kWideStages;
+                if (!mbar_wait(&empty[s], ((it / kWideStages) & 1) ^ 1)) {
+                    if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                    alive = false;
+                    break;
+                }
+                if (elect_one()) {
+                    if (it >= ahead) request_weights(s, i, group.x, n0, width, boxes);
+                    uint8_t* planes = smem + s * kWideStageBytes + 2 * kWeightBytes;
+                    for (int b = 0; b < boxes; ++b) {
+                        tma_load_2d(planes + b * kBoxBytes, &map_hi, i * kBlockK, group.y + b * kBox, &full[s]);
+                        tma_load_2d(planes + kWidePlaneBytes + b * kBoxBytes, &map_lo, i * kBlockK, group.y + b * kBox, &full[s]);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp == 1) {
+        int it = 0, j = 0;
+        bool alive = true;
+        for (int unit = blockIdx.x; unit < w.units && alive; unit += gridDim.x, ++j) {
+            int row_tile, n0, width;
+            w.place(unit, p.out, row_tile, n0, width);
+            const uint32_t instruction = width == kWideN ? kWhole : kHalf, accumulator = tmem_base + static_cast<uint32_t>((j & 1) * kWideN);
+            // the epilogue of the tile that used this buffer two tiles ago must have read it (passes at once for j < 2)
+            if (!mbar_wait(&acc_empty[j & 1], ((j >> 1) & 1) ^ 1)) {
+                if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                break;
+            }
+            tc_fence_after_sync();
+            for (int i = 0; i < k_blocks; ++i, ++it) {
+                const int s = it % kWideStages;
+                if (!mbar_wait(&full[s], (it / kWideStages) & 1)) {
+                    if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                    alive = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                if (elect_one()) {
+                    const uint32_t stage = smem_u32(smem + s * kWideStageBytes);
+                    const uint64_t weights = operand_descriptor(stage), hi = operand_descriptor(stage + 2 * kWeightBytes);
+                    const uint64_t lo = operand_descriptor(stage + 2 * kWeightBytes + kWidePlaneBytes);
+#pragma unroll
+                    for (int k = 0; k < kBlockK / 16; ++k) {
+                        tc_mma_bf16(accumulator, hi + 2 * k, weights + 2 * k, instruction, (i | k) != 0);
+                        tc_mma_bf16(accumulator, lo + 2 * k, weights + 2 * k, instruction, 1);
+                    }
+                    tc_commit(&empty[s]);
+                    if (i == k_blocks - 1) tc_commit(&acc_full[j & 1]);
+                }
+                __syncwarp();
+            }
+        }
+    } else {
+        // ---- epilogue warps 2-9: TMEM lanes 32 * (warp % 4) .. + 31, features [128 * half, + 128) of the tile ----
+        const int quarter = warp & 3, half = (warp - 2) >> 2, tile_row = quarter * 32 + lane;
+        int j = 0;
+        for (int unit = blockIdx.x; unit < w.units; unit += gridDim.x, ++j) {
+            int row_tile, n0, width;
+            w.place(unit, p.out, row_tile, n0, width);
+            const int4 group = __ldg(gp.tiles + row_tile);
+            const int slot = tile_row < group.z ? group.y + tile_row : p.rows;   // rows past the group's hold no results
+            const float scale = gp.scale && tile_row < group.z ? __ldg(gp.scale + slot) : 1.0f;
+            if (!mbar_wait_relaxed(&acc_full[j & 1], (j >> 1) & 1)) {
+                if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                break;
+            }
+            tc_fence_after_sync();
+            if (half * kTile < width && quarter * 32 < group.z) {
+                const uint32_t address = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>((j & 1) * kWideN + half * kTile);
+                float squares = 0.0f;
+#pragma unroll 1
+                for (int c = 0; c < kTile; c += 32) finish_chunk<EPI>(p, slot, n0 + half * kTile + c, address + c, scale, make_int2(0, 0), squares);
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[j & 1]);
+        }
+    }
+    __syncwarp();
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, 2 * kWideN);
+    }
+}
+
 // One CTA per row: y = residual + the row's results in the order of its choices.  FINISH: the sum goes through the norm behind the mixture.
 template <bool FINISH>
 __global__ void __launch_bounds__(256) expert_combine_kernel(const __grid_constant__ ExpertParams p, const float* results, const int32_t* place) {
@@ -593,10 +775,15 @@ int launch_expert_gemm(const ExpertParams& e, const Grouped& g, const __nv_bfloa
     gp.base.rows = slots; gp.base.in = in; gp.base.out = out;
     gp.tiles = g.tiles; gp.tile_count = g.tile_count;
     const int ctas = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(most_tiles(e)) * ((out + kTile - 1) / kTile), sms));
+    if (tile_slots(e) == kTile) {   // (what its epilogue stores lies in the workspace, on 16-byte borders)
+        auto kernel = expert_gemm_wide_kernel<EPI>;
+        B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmem));
+        return cuda_status(launch_dependent(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kWideThreads), kWideSmem, stream, map_hi, map_lo, map_w, gp),
+                           "expert_gemm_wide_kernel launch");
+    }
     switch (tile_slots(e)) {
     case 32: return launch_expert_tiles<EPI, 32>(map_hi, map_lo, map_w, gp, ctas, stream);
-    case 64: return launch_expert_tiles<EPI, 64>(map_hi, map_lo, map_w, gp, ctas, stream);
-    default: return launch_expert_tiles<EPI, 128>(map_hi, map_lo, map_w, gp, ctas, stream);
+    default: return launch_expert_tiles<EPI, 64>(map_hi, map_lo, map_w, gp, ctas, stream);
     }
 }
 

@@ -552,7 +552,8 @@ def test_dense_tensor_core_linear(rows, inner, out, epilogue):
                                                      (1024, 520, 2080, 1),    # all tiles in halves
                                                      (2100, 2056, 2144, 1),   # K beyond the persistent kernel's, a ragged last row tile
                                                      (1024, 136, 4160, 2),
-                                                     (1030, 64, 5000, 0)])    # features that are no multiple of 32: not this kernel
+                                                     (1030, 64, 5000, 0), (1100, 96, 2312, 1), (1024, 64, 4112, 2),   # features that end inside a chunk of 32
+                                                     (1024, 64, 4100, 0)])    # no multiple of 8: not this kernel
 def test_wide_linear_tiles(rows, inner, out, epilogue):
     """Passes of eight or more token tiles on tiles of 128 x 256: bands, halves of the last round, ragged edges."""
     test_dense_tensor_core_linear(rows, inner, out, epilogue)

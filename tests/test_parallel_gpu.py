@@ -303,6 +303,12 @@ def test_grouped_experts(rows, experts, top, width, ff, load):
     assert run_experts(rows, experts, top, width, ff, "bf16", "grouped", load) < 5e-5
 
 
+@pytest.mark.parametrize("rows, experts, top, width, ff", [(1500, 6, 2, 520, 1032), (260, 3, 1, 264, 72), (400, 4, 2, 1000, 40)])
+def test_grouped_experts_on_wide_tiles(rows, experts, top, width, ff):
+    """Row tiles of 128 slots, some of them short; whole tiles of 256 features and halves in the last round, widths that end inside a chunk of 32."""
+    assert run_experts(rows, experts, top, width, ff, "bf16", "grouped", "some") < 5e-5
+
+
 @pytest.mark.parametrize("rows, inner, units", [(1, 64, 40), (16, 256, 130), (40, 136, 64), (300, 128, 100), (270, 64, 33)])
 def test_gated_units_beside_other_columns(rows, inner, units):
     """SwiGLU epilogue into a column range of wider rows, every linear kernel family."""
