@@ -396,6 +396,30 @@ def test_shadow_protocol_norm_linear_residual(rows, inner, out):
     assert rel(osq.cpu().numpy().sum(axis=0), (want.astype(np.float64) ** 2).sum(axis=1)) < 1e-4
 
 
+@pytest.mark.parametrize("width", [1, 4, 1030, 4096, 4100, 8196])
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+def test_embedding_rows_and_planes(width, dtype):
+    """Embedding rows with their planes and sums of squares: single values and fours, a thread's last batch partly past the end, two batches."""
+    l = B.lib()
+    g = torch.Generator(device="cuda").manual_seed(width)
+    kind = torch.bfloat16 if dtype == "bf16" else torch.float32
+    table = torch.randn((7, width), generator=g, device="cuda").to(kind)
+    norm = (1 + 0.1 * torch.randn(width, generator=g, device="cuda")).to(kind)
+    ids = torch.tensor([6, 0, 3], device="cuda")
+    out = torch.full((3, width), float("nan"), device="cuda")
+    hi, lo = (torch.full((3, width), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    squares = torch.empty(3, device="cuda")
+    code = B.BF16 if dtype == "bf16" else B.F32
+    torch.cuda.synchronize()
+    B.kcheck(l.b200_embedding_shadow(table.data_ptr(), code, ids.data_ptr(), 3, 7, width, norm.data_ptr(), code, out.data_ptr(), hi.data_ptr(),
+                                     lo.data_ptr(), squares.data_ptr(), stream()))
+    sync()
+    x = table[ids].float()
+    scaled = x * norm.float()
+    assert torch.equal(out, x) and torch.equal(hi, scaled.bfloat16()) and torch.equal(lo, (scaled - scaled.bfloat16().float()).bfloat16())
+    assert torch.allclose(squares.double(), x.double().square().sum(1), rtol=1e-5)
+
+
 @pytest.mark.parametrize("rows,inner,out", [(1, 8, 2), (1, 2048, 3072), (4, 14336, 4096), (3, 4104, 1001), (8, 2040, 16), (9, 1032, 2369 * 2), (16, 768, 32000), (13, 40, 130)])
 def test_streaming_linear_at_the_edges_of_its_tiles(rows, inner, out):
     """Shadow linears of at most 16 rows: 8 | 9 rows (one or two token tiles), chunks of 32 columns and tiles of 16 features that end early, fewer
