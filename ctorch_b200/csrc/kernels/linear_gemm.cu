@@ -581,10 +581,11 @@ int choose_tile_features(int rows, int in, int out) {
     return row_tiles * ((out + 255) / 256) >= 2 * sms ? 256 : 128;
 }
 
-// Ring depth for the 128-wide tile: two stages (96 KB) let two CTAs share an SM, so one tile's epilogue and pipeline ramp
-// overlap the other's products; up to 64 rows the activation boxes are mostly zero fill and a CTA alone with a deep ring
-// streams weights faster.
-int choose_stages(int rows) { return rows > 64 ? 2 : 4; }
+// Ring depth for the 128-wide tile: two stages (96 KB) let two CTAs share an SM, so one tile's epilogue and pipeline ramp overlap the other's
+// products; where there is no second CTA for every SM, and up to 64 rows, whose activation boxes are mostly zero fill, a CTA alone with
+// a deep ring streams faster (8192 -> 2048 at 844 rows 98 us with two stages, 67 with four; 4096 -> 1024 at 1500 rows 51 and 39).  Not with a
+// K split: clusters of CTAs that each fill an SM place badly (8192 -> 2048 at 300 rows 40 us with two stages, 51 with four).
+int choose_stages(int rows, int64_t tiles, int split, int sms) { return rows > 64 && (split > 1 || tiles > sms) ? 2 : 4; }
 
 // K split of a launch: cluster CTAs (grid z) while the grid stays within one wave of the SMs, at most 4 (larger clusters
 // of CTAs this big place badly), and at least two K blocks per CTA.
@@ -702,7 +703,7 @@ int launch_linear_gemm(const LinearParams& p, int epilogue, cudaStream_t stream)
     if (status == B200_OK) status = encode_operand(&w, p.weight, p.out, p.in, tn);
     if (status != B200_OK) return status;
     if (persistent) return launch_persistent(epilogue, hi, lo, w, gp, row_tiles, tiles128, sms, stream);
-    const int stages = choose_stages(p.rows);
+    const int stages = choose_stages(p.rows, tiles128, choose_split(p.rows, p.in, p.out), sms);
     if (tn == 256) return launch_epilogue<256, 3>(epilogue, hi, lo, w, gp, stream);
     return stages == 2 ? launch_epilogue<128, 2>(epilogue, hi, lo, w, gp, stream) : launch_epilogue<128, 4>(epilogue, hi, lo, w, gp, stream);
 }
