@@ -23,7 +23,9 @@
 #include "kv_cache.cuh"
 
 #include <cmath>
+#include <map>
 #include <mutex>
+#include <utility>
 
 namespace b200 {
 namespace {
@@ -136,8 +138,8 @@ constexpr int kMostClustered = 8;   // CTAs of a cluster, the largest portable s
 
 // MULTI: items of several positions (prefill chunks); the decode instantiation keeps one position per item and one key
 // count for all of its rows.
-// CLUSTERED: the splits of an item (grid y) are a thread-block cluster that merges them through distributed shared memory; every CTA
-// stays to the end, with pages or without.
+// CLUSTERED: the splits of an item (grid y) are a thread-block cluster that merges them through distributed shared memory, in the order and
+// arithmetic of attention_combine_kernel; every CTA stays to the end, with pages or without.
 template <int HD, int STAGES, bool MULTI, bool CLUSTERED>
 __global__ void __launch_bounds__(kFastThreads) attention_mma_kernel(const __grid_constant__ CUtensorMap kmap,
                                                                      const __grid_constant__ CUtensorMap vmap,
@@ -164,8 +166,8 @@ __global__ void __launch_bounds__(kFastThreads) attention_mma_kernel(const __gri
     const int base_len = p.kv.lengths[sequence];
     const int kv_len = base_len + (p.causal ? t_first + t_count : 0);   // keys the item's last position sees
     int page_end = (kv_len + kFastPageSize - 1) / kFastPageSize;
-    const int per_split = CLUSTERED ? (page_end + static_cast<int>(gridDim.y) - 1) / static_cast<int>(gridDim.y)
-                                    : balanced_pages_per_split(page_end, p.pages_per_split);
+    const int per_split = balanced_pages_per_split(page_end, p.pages_per_split);
+    const int filled = CLUSTERED ? min((page_end + per_split - 1) / per_split, static_cast<int>(gridDim.y)) : 0;   // splits that have pages
     const int page_begin = split * per_split;
     if (page_end > page_begin + per_split) page_end = page_begin + per_split;
     if (!CLUSTERED && page_begin >= page_end) return;  // uniform for the CTA
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(kFastThreads) attention_mma_kernel(const __gri
             float2 ml[kMostClustered];
 #pragma unroll
             for (int c = 0; c < kMostClustered; ++c) {
-                const bool there = c < static_cast<int>(gridDim.y);
+                const bool there = c < filled;
                 const uint32_t pair = map_peer_shared(ml_at + r * 8, there ? c : 0), at = map_peer_shared(o_at + i * 4, there ? c : 0);
                 ml[c] = there ? make_float2(load_cluster_float(pair), load_cluster_float(pair + 4)) : make_float2(-INFINITY, 0.0f);
                 value[c] = there ? load_cluster_float(at) : 0.0f;
@@ -393,11 +395,12 @@ __global__ void __launch_bounds__(kFastThreads) attention_mma_kernel(const __gri
             for (int c = 0; c < kMostClustered; ++c) m = fmaxf(m, ml[c].x);
 #pragma unroll
             for (int c = 0; c < kMostClustered; ++c) {
-                const float weight = ml[c].x == -INFINITY ? 0.0f : expf(ml[c].x - m);
-                acc += weight * value[c];
-                l += weight * ml[c].y;
+                if (c >= filled) break;
+                l += expf(ml[c].x - m) * ml[c].y;
+                acc += expf(ml[c].x - m) * value[c];
             }
-            store_result(p, (static_cast<int64_t>(row) * p.heads + kvh * group + r) * HD + d, acc / l);
+            // (a row that sees no key is left as it is)
+            if (filled > 0) store_result(p, (static_cast<int64_t>(row) * p.heads + kvh * group + r) * HD + d, acc / l);
         }
         cluster_sync_all();   // nobody leaves while a peer reads its shared memory
     }
@@ -950,6 +953,7 @@ __global__ void attention_combine_kernel(const AttnParams p) {
     const int per_split = balanced_pages_per_split(pages, p.pages_per_split);
     int valid = (pages + per_split - 1) / per_split;   // splits whose CTA had pages and wrote a partial
     if (valid > p.num_splits) valid = p.num_splits;
+    if (valid == 0) return;   // a row that sees no key is left as it is, as without splits
     const float* ml = p.part_ml + head_item * p.num_splits * 2;
     float m = -INFINITY;
     for (int s = 0; s < valid; ++s) m = fmaxf(m, ml[2 * s]);
@@ -960,17 +964,6 @@ __global__ void attention_combine_kernel(const AttnParams p) {
         for (int s = 0; s < valid; ++s) acc += expf(ml[2 * s] - m) * p.part_o[(head_item * p.num_splits + s) * hd + d];
         store_result(p, head_item * hd + d, acc / l);
     }
-}
-
-// CTAs per item (sequence, KV head) of a decode launch that merges inside a cluster; 1: none.  Few items leave SMs idle and a merge kernel costs
-// a launch, so the largest cluster that keeps all CTAs resident (two per SM at head_dim 64, whose smaller ring allows it) and gives each
-// two pages; contexts of more than 16 pages per CTA go to the split plan, whose CTAs are as many as the pages ask for.  Measured inside
-// decode steps, attention and merge kernel before -> one launch: 64 items of 9 pages 9.5 -> 6.9 us, 8 items of 24 pages 9.3 -> 6.0 us.
-int cluster_size(int64_t items, int pages, int head_dim, int sms) {
-    const int64_t slots = head_dim == 64 ? 2 * sms : sms;
-    for (int c = kMostClustered; c > 1; c >>= 1)
-        if (items * c <= slots && pages >= 2 * c) return pages <= 16 * c ? c : 1;
-    return 1;
 }
 
 // Whether a pass takes the prefill kernel: at least three of its eight warps have rows (below that, attention_mma_kernel's warps, which share
@@ -992,7 +985,33 @@ template <int HD> int launch_prefill(const b200_kv_cache* cache, AttnParams p, c
                                         *kv_tensor_map(cache, 1), p), "attention_prefill_kernel launch");
 }
 
-template <int HD, int STAGES> int launch_fast(const b200_kv_cache* cache, AttnParams p, int clustered, cudaStream_t stream) {
+// Clusters of `splits` CTAs that the device holds at once; asked of the runtime once per device and size, and kept.
+template <int HD, int STAGES> int resident_clusters(int splits, int device) {
+    static std::mutex mutex;
+    static std::map<std::pair<int, int>, int> known;
+    std::lock_guard<std::mutex> lock(mutex);
+    const auto [at, first] = known.try_emplace({device, splits}, 0);
+    if (!first) return at->second;
+    auto kernel = attention_mma_kernel<HD, STAGES, false, true>;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(1, static_cast<unsigned>(splits));
+    config.blockDim = dim3(kFastThreads);
+    config.dynamicSmemBytes = FastShape<HD, STAGES>::smem_bytes;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = 1; attribute.val.clusterDim.y = static_cast<unsigned>(splits); attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FastShape<HD, STAGES>::smem_bytes) != cudaSuccess
+        || cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+        cudaGetLastError();
+        clusters = 0;
+    }
+    return at->second = clusters;
+}
+
+template <int HD, int STAGES> int launch_fast(const b200_kv_cache* cache, AttnParams p, bool& merged, cudaStream_t stream) {
     using S = FastShape<HD, STAGES>;
     const int blocks_per_sequence = (p.tokens_per_sequence + p.positions_per_item - 1) / p.positions_per_item;
     const int items = (p.rows / p.tokens_per_sequence) * blocks_per_sequence * p.kv.kv_heads;
@@ -1002,9 +1021,21 @@ template <int HD, int STAGES> int launch_fast(const b200_kv_cache* cache, AttnPa
     const int group = p.heads / p.kv.kv_heads;
     const int merge_bytes = kConsumerWarps * group * (HD + 2) * static_cast<int>(sizeof(float));
     const int persist_bytes = S::smem_bytes + merge_bytes;   // the merge area follows the control block
+    // Splits of decode items merge inside a cluster where the device holds all of them at once: the merge kernel's launch and the partials' way through
+    // memory are saved (8 items of 24 pages, three splits, inside a decode step: 9.3 -> 7.5 us); a second wave would cost more than that.
+    if (p.num_splits > 1 && p.num_splits <= kMostClustered && p.positions_per_item == 1 && p.tokens_per_sequence == 1
+        && items <= resident_clusters<HD, STAGES>(p.num_splits, device)) {
+        auto kernel = attention_mma_kernel<HD, STAGES, false, true>;
+        B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::smem_bytes));
+        const unsigned splits = static_cast<unsigned>(p.num_splits);
+        merged = true;
+        return cuda_status(launch_dependent_cluster(kernel, dim3(static_cast<unsigned>(items), splits), dim3(kFastThreads), S::smem_bytes, stream,
+                                                    dim3(1, splits, 1), *kv_tensor_map(cache, 0), *kv_tensor_map(cache, 1), p),
+                           "attention_mma_kernel launch");
+    }
     // With split items the units are dealt out in turn, which only balances when the sequences are equally long (what
     // the cache's owner knows on the host); ragged split batches keep one CTA per unit and the hardware's scheduling.
-    if (clustered <= 1 && p.positions_per_item == 1 && persist_bytes <= 232448 && static_cast<int64_t>(items) * p.num_splits > sm_count(device)
+    if (p.positions_per_item == 1 && persist_bytes <= 232448 && static_cast<int64_t>(items) * p.num_splits > sm_count(device)
         && (p.num_splits == 1 || cache->even_lengths)) {
         auto kernel = attention_persistent_kernel<HD, STAGES>;
         B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, persist_bytes));
@@ -1023,14 +1054,6 @@ template <int HD, int STAGES> int launch_fast(const b200_kv_cache* cache, AttnPa
         p.items = items;
         return cuda_status(launch_dependent(kernel, dim3(static_cast<unsigned>(resident)), dim3(kFastThreads), static_cast<size_t>(persist_bytes),
                                             stream, *kv_tensor_map(cache, 0), *kv_tensor_map(cache, 1), p), "attention_mma_kernel launch");
-    }
-    if (clustered > 1) {
-        auto kernel = attention_mma_kernel<HD, STAGES, false, true>;
-        B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::smem_bytes));
-        const unsigned splits = static_cast<unsigned>(clustered);
-        return cuda_status(launch_dependent_cluster(kernel, dim3(static_cast<unsigned>(items), splits), dim3(kFastThreads), S::smem_bytes, stream,
-                                                    dim3(1, splits, 1), *kv_tensor_map(cache, 0), *kv_tensor_map(cache, 1), p),
-                           "attention_mma_kernel launch");
     }
     auto kernel = p.positions_per_item > 1 ? attention_mma_kernel<HD, STAGES, true, false> : attention_mma_kernel<HD, STAGES, false, false>;
     B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::smem_bytes));
@@ -1086,10 +1109,6 @@ int attention_launch(const float* q, int64_t rows, int32_t tokens_per_sequence, 
         set_error("b200_attention_decode: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
         return B200_BAD_ARGUMENT;
     }
-    int device = 0;
-    B200_CUDA(cudaGetDevice(&device));
-    const int clustered = fast && tokens_per_sequence == 1 ? cluster_size(rows * cache->kv_heads, plan.pages_total, cache->head_dim, sm_count(device)) : 1;
-    if (clustered > 1) plan.num_splits = 1;   // merged inside the kernel: no partials in the scratch
     AttnParams p{};
     p.q = q; p.rows = static_cast<int>(rows); p.tokens_per_sequence = tokens_per_sequence; p.heads = heads; p.causal = causal;
     p.positions_per_item = positions;
@@ -1103,24 +1122,27 @@ int attention_launch(const float* q, int64_t rows, int32_t tokens_per_sequence, 
     if (!p.status) { set_error("b200_attention_decode: the device status word could not be allocated"); return B200_NO_DEVICE; }
     cudaStream_t s = as_stream(stream);
     int status;
+    bool merged = plan.num_splits == 1;   // nothing is left to the merge kernel
     if (fast) {
+        int device = 0;
+        B200_CUDA(cudaGetDevice(&device));
         // head_dim 64 with more CTAs than SMs: a 96 KB ring lets two CTAs share an SM, so one CTA's pipeline ramp and
         // drain overlap the other's streaming; with fewer CTAs each keeps the deeper ring to itself.
-        const int64_t ctas = clustered * (static_cast<int64_t>(p.rows) / tokens_per_sequence) * ((tokens_per_sequence + positions - 1) / positions)
+        const int64_t ctas = (static_cast<int64_t>(p.rows) / tokens_per_sequence) * ((tokens_per_sequence + positions - 1) / positions)
                              * p.kv.kv_heads * p.num_splits;
         // pairs of results are stored together: the planes and rows that callers hand in are 4- and 8-byte aligned for that
         const bool pairs = ((out_hi ? (reinterpret_cast<uintptr_t>(out_hi) | reinterpret_cast<uintptr_t>(out_lo)) << 1 : reinterpret_cast<uintptr_t>(out)) & 7) == 0;
         if (tokens_per_sequence > 1 && pairs && takes_prefill(tokens_per_sequence, group, ctas, plan.pages_total, cache->head_dim, sm_count(device)))
             return cache->head_dim == 128 ? launch_prefill<128>(cache, p, s) : launch_prefill<64>(cache, p, s);
-        if (cache->head_dim == 128) status = launch_fast<128, 6>(cache, p, clustered, s);
-        else if (ctas > sm_count(device)) status = launch_fast<64, 6>(cache, p, clustered, s);
-        else status = launch_fast<64, 8>(cache, p, clustered, s);
+        if (cache->head_dim == 128) status = launch_fast<128, 6>(cache, p, merged, s);
+        else if (ctas > sm_count(device)) status = launch_fast<64, 6>(cache, p, merged, s);
+        else status = launch_fast<64, 8>(cache, p, merged, s);
     } else {
         const dim3 grid(static_cast<unsigned>(rows) * heads, plan.num_splits);
         status = cuda_status(launch_dependent(attention_generic_kernel, grid, dim3(kGenericThreads), sizeof(float) * kGenericWarps * cache->head_dim, s, p),
                              "attention_generic_kernel launch");
     }
-    if (status != B200_OK || plan.num_splits == 1) return status;
+    if (status != B200_OK || merged) return status;
     return cuda_status(launch_dependent(attention_combine_kernel, dim3(static_cast<unsigned>(rows) * heads), dim3(128), 0, s, p),
                        "attention_combine_kernel launch");
 }

@@ -260,10 +260,12 @@ def test_decode_attention_ragged(cache_dtype, hd, heads, kv_heads, lengths):
 
 
 @pytest.mark.parametrize("cache_dtype,hd,heads,kv_heads,lengths", [
-    (B.BF16, 64, 8, 2, [1024, 64, 1, 513]),            # clusters of eight, some of whose CTAs have no page
-    (B.BF16, 128, 16, 1, [8192, 65]),                  # eight CTAs of 16 pages
-    (B.BF16, 128, 16, 1, [8193, 4000]),                # one page more: the split plan and its merge kernel
-    (B.BF16, 64, 12, 4, [100 + 37 * s for s in range(16)]),   # four per item
+    (B.BF16, 64, 8, 2, [1024, 64, 1, 513]),            # 16 pages: no splits
+    (B.BF16, 64, 8, 2, [1025, 64, 1, 513]),            # 17 pages: clusters of three, some of whose CTAs have no page
+    (B.BF16, 128, 8, 2, [4096, 65, 2000]),             # clusters of eight
+    (B.BF16, 128, 16, 1, [8192, 65]),                  # sixteen splits: the merge kernel
+    (B.BF16, 128, 16, 1, [8193, 4000]),
+    (B.BF16, 64, 12, 4, [100 + 37 * s for s in range(16)]),
     (B.F32, 256, 4, 2, [7, 8, 9, 63, 64, 65]),         # generic path: batches of eight tokens that end early
     (B.F32, 40, 3, 1, [1, 129]),
     (B.BF16, 64, 20, 1, [70, 2000]),                   # 20 heads on one cached head: generic path on a bf16 pool, split
@@ -271,6 +273,41 @@ def test_decode_attention_ragged(cache_dtype, hd, heads, kv_heads, lengths):
 def test_decode_attention_of_few_items(cache_dtype, hd, heads, kv_heads, lengths):
     """Launches with fewer items than SMs: splits merged inside a cluster, and the generic kernel's batches of tokens."""
     test_decode_attention_ragged(cache_dtype, hd, heads, kv_heads, lengths)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_decode_results_do_not_hang_on_the_batch(hd):
+    """Four sequences by themselves, whose splits merge inside clusters, and the same four among 54, whose clusters the device does not hold at once
+    (the merge kernel): the split plan is the same for both, and so are the results, bit for bit."""
+    rng = np.random.default_rng(hd)
+    lengths, heads, kv_heads, cap = [2500, 513, 1, 1600], 8, 2, 2500
+    k, v = (rng.standard_normal((54, kv_heads, cap, hd), dtype=np.float32) for _ in range(2))
+    q = rng.standard_normal((54, heads, hd), dtype=np.float32)
+    got = []
+    for n in (4, 54):
+        cache = Cache(B.BF16, n, kv_heads, hd, cap)
+        cache.append(k[:n], v[:n])
+        cache.set_lengths(np.array((lengths * 14)[:n], dtype=np.int32) - 1)
+        got.append(attention(q[:n], cache, 1, heads, cap)[:4])
+    assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("hd,n,cap,L", [(64, 4, 2500, 1), (64, 54, 2500, 1), (64, 4, 300, 1), (64, 4, 300, 40), (32, 4, 2500, 1)])
+def test_rows_that_see_no_key_are_left_alone(hd, n, cap, L):
+    """Not causal, an empty sequence: splits merged inside a cluster and by the merge kernel, no splits, many positions, the generic kernel."""
+    rng = np.random.default_rng(hd + n)
+    cache = Cache(B.BF16, n, 2, hd, cap)
+    k, v = (rng.standard_normal((n, 2, cap, hd), dtype=np.float32) for _ in range(2))
+    cache.append(k, v)
+    cache.set_lengths(np.array([0, cap] * (n // 2), dtype=np.int32))
+    q = torch.randn((n * L, 8, hd), device="cuda")
+    need = B.lib().b200_attention_scratch_bytes(n * L, 8, 2, hd, cap, 64)
+    scratch = torch.empty((need,), dtype=torch.uint8, device="cuda")
+    out = torch.full((n, L, 8 * hd), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    B.kcheck(B.lib().b200_attention_decode(q.data_ptr(), n * L, L, 8, cache.h, cap, 0, scratch.data_ptr(), need, out.data_ptr(), stream()))
+    sync()
+    assert bool((out[0::2] == 7.0).all()) and bool((out[1::2].abs() < 5.0).all())
 
 
 @pytest.mark.parametrize("cache_dtype,hd", [(B.F32, 32), (B.BF16, 64)])
