@@ -98,13 +98,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// 2^v by the hardware unit (relative error about 2^-22; 2^-inf = 0)
-__device__ __forceinline__ float exp2_fast(float v) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return r;
-}
-
 constexpr int kConsumerWarps = 8;   // two groups of four: group g takes pages g, g+2, ... so two pages are in the
 constexpr int kGroupWarps = 4;      // tensor-core pipeline at a time; a warp owns 16 tokens of its group's page
 constexpr int kFastThreads = (kConsumerWarps + 1) * 32;
@@ -659,49 +652,64 @@ __global__ void __launch_bounds__(kFastThreads) attention_persistent_kernel(cons
     }
 }
 
-// Passes of many positions per sequence (prefill): 128 fragment rows per CTA - consecutive positions times the head group - of which each of
-// the eight warps takes 16 through all pages, so a page that is staged once serves all of them and no sums are merged in the end.
-// Products and precision are those of attention_mma_kernel (bf16 q and weights, f32 scores, softmax and sums).  Bound by the instruction
-// issue of mma.sync and the softmax around it.  Blocks of late positions, which see the most pages, come first.  8 prompts of 1024
-// positions, 32 / 8 heads of 64: attention_mma_kernel, whose CTAs take 16 rows and share out each page's tokens, 598 us (57 TFLOP/s useful),
-// this one 149 (230); 2 of 4096 positions, heads of 128: 2618 and 882 us (312 TFLOP/s).
-constexpr int kPrefillRows = kConsumerWarps * 16, kPrefillThreads = kConsumerWarps * 32;
-template <int HD> constexpr int prefill_stages() { return HD == 64 ? 5 : 4; }   // 80 KB: two CTAs per SM; 128 KB: one
+// Passes of many positions per sequence (prefill): the arithmetic of attention_mma_kernel - a warp takes 16 tokens of every second page, with a running
+// maximum, sum and accumulator of its own, and the eight of them are merged in the end, so that a row's result does not hang on the
+// kernel, bit for bit - for two blocks of 16 fragment rows per CTA: a page is staged and its fragments are fetched once for both, whose
+// chains of dependent instructions run side by side.  Every row sees the keys of its own position: a page behind those adds nothing.
+// Blocks of late positions, which see the most pages, come first.  Bound by the chain of a page (products, softmax, products), of which 16 warps
+// per SM (8 with heads of 128) hide a part, and by what stands around the pages, 5 us of a CTA's 14 at 1024 positions.  us, attention_mma_kernel
+// | here: 8 prompts of 1024 positions, 32 / 8 heads of 64 598 | 388; 16 of 549, 12 / 4 heads 207 | 127; 2 of 4096, heads of 128 2619 | 2146.
+// (With 16 rows per warp through whole pages, 128 a CTA, the first took 149 us, but then the weights, rounded to bf16, are relative to one maximum
+// instead of eight: 18 % further from 64 bits, with peaked scores twice as far.)
+constexpr int kPrefillThreads = kConsumerWarps * 32, kPrefillBlocks = 2, kPrefillStages = 6;   // 96 KB of pages: two CTAs per SM; 192 KB: one
+template <int HD> struct PrefillShape : FastShape<HD, kPrefillStages> {
+    using Base = FastShape<HD, kPrefillStages>;
+    static constexpr int q_bytes = kPrefillBlocks * (HD / 16) * 32 * 16;   // q as fragments of the products
+    static constexpr int smem_bytes = Base::smem_bytes + q_bytes;
+    static constexpr int pitch = HD + 8;   // merge area: [blocks][warps][16][pitch], then (max, sum) and weights
+    static constexpr int units = kPrefillBlocks * kConsumerWarps * 16;
+    static_assert(units * (pitch + 3) * 4 + kPrefillBlocks * 16 * 4 <= Base::stages * Base::stage_bytes);
+};
 
 template <int HD>
 __global__ void __launch_bounds__(kPrefillThreads, HD == 64 ? 2 : 1) attention_prefill_kernel(const __grid_constant__ CUtensorMap kmap,
                                                                                            const __grid_constant__ CUtensorMap vmap, const AttnParams p) {
-    using S = FastShape<HD, prefill_stages<HD>()>;
+    using S = PrefillShape<HD>;
     extern __shared__ uint8_t smem_raw[];
+    __shared__ int gave_up;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::stages * S::stage_bytes);
     uint64_t* empty = full + S::stages;
+    uint4* q_fragments = reinterpret_cast<uint4*>(smem + S::stages * S::stage_bytes + kFastControlBytes);   // [blocks][HD / 16][lanes]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::stages; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&empty[s], kConsumerWarps);
+            mbar_init(&empty[s], kGroupWarps);
         }
+        gave_up = 0;
         mbar_fence_init();
     }
     __syncthreads();
     grid_dependency_wait();   // q, the cache and the lengths come from the preceding kernels
     grid_launch_dependents();
 
-    const int group = p.heads / p.kv.kv_heads, positions = p.positions_per_item;
+    const int group = p.heads / p.kv.kv_heads, positions = p.positions_per_item, span = kPrefillBlocks * positions;
     const int streams = p.kv.sequences * p.kv.kv_heads;   // (sequence, KV head)
-    const int blocks = (p.tokens_per_sequence + positions - 1) / positions;
-    const int stream = blockIdx.x % streams, block = blocks - 1 - static_cast<int>(blockIdx.x) / streams;
+    const int spans = (p.tokens_per_sequence + span - 1) / span;
+    const int stream = blockIdx.x % streams, t_first = (spans - 1 - static_cast<int>(blockIdx.x) / streams) * span;
     const int sequence = stream / p.kv.kv_heads, kvh = stream - sequence * p.kv.kv_heads;
-    const int t_first = block * positions, t_count = min(positions, p.tokens_per_sequence - t_first);
+    const int t_count = min(span, p.tokens_per_sequence - t_first);
     const int base_len = p.kv.lengths[sequence];
     const int pages = (base_len + (p.causal ? t_first + t_count : 0) + kFastPageSize - 1) / kFastPageSize;
+    if (pages == 0) return;   // a row that sees no key is left as it is
 
     // The first lane of warp 0 requests the pages: a ring's worth here, later ones kLag pages after their stage was last read.
-    constexpr int kLag = 2;
+    constexpr int kLag = 4;
     const int32_t* table = p.kv.page_table + static_cast<int64_t>(sequence) * p.kv.pages_per_seq;
-    auto request = [&](int i) {
-        const int s = i % S::stages, y = (table[i] * p.kv.kv_heads + kvh) * kFastPageSize;
+    int requested = 0;
+    auto request = [&] {
+        const int s = requested % S::stages, y = (table[requested] * p.kv.kv_heads + kvh) * kFastPageSize;
         uint8_t* kdst = smem + s * S::stage_bytes;
         uint8_t* vdst = kdst + S::tile_bytes;
         mbar_expect_tx(&full[s], S::stage_bytes);
@@ -710,128 +718,193 @@ __global__ void __launch_bounds__(kPrefillThreads, HD == 64 ? 2 : 1) attention_p
             tma_load_2d(kdst + h * kHalfTileBytes, &kmap, h * 64, y, &full[s]);
             tma_load_2d(vdst + h * kHalfTileBytes, &vmap, h * 64, y, &full[s]);
         }
+        ++requested;
     };
     if (threadIdx.x == 0)
-        for (int i = 0; i < min(pages, S::stages); ++i) request(i);
+        while (requested < min(pages, S::stages)) request();
 
-    // ---- this thread's two fragment rows, their activation rows and the keys each sees ----
     const int g = lane >> 2, t = lane & 3, mi = lane >> 3, ri = lane & 7;
-    int limit[2], at_row[2], at_head[2];
-    bool live[2];
-    uint32_t qa[HD / 16][4];
+    // fragment row r of block b: position b * positions + r / group, query head r % group
+    auto rows_of = [&](int b) { return group * max(0, min(positions, t_count - b * positions)); };
+    auto row_at = [&](int b, int r) {
+        const int position = r / group;
+        return (static_cast<int64_t>(sequence) * p.tokens_per_sequence + t_first + b * positions + position) * p.heads + kvh * group + (r - position * group);
+    };
+    for (int f = warp; f < kPrefillBlocks * (HD / 16); f += kConsumerWarps) {
+        const int b = f / (HD / 16), c = (f - b * (HD / 16)) * 16 + 2 * t;
+        uint32_t q[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int r = warp * 16 + g + 8 * h, position = r / group;
-        live[h] = r < group * t_count;
-        at_row[h] = sequence * p.tokens_per_sequence + t_first + position;
-        at_head[h] = kvh * group + (r - position * group);
-        limit[h] = live[h] ? base_len + (p.causal ? t_first + position + 1 : 0) : 0;
-        const float* q = p.q + (static_cast<int64_t>(at_row[h]) * p.heads + at_head[h]) * HD;
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-            const int c = kk * 16 + 2 * t;
-            qa[kk][h] = live[h] ? pack_bf16(q[c], q[c + 1]) : 0u;
-            qa[kk][2 + h] = live[h] ? pack_bf16(q[c + 8], q[c + 9]) : 0u;
-        }
+        for (int h = 0; h < 2; ++h)
+            if (g + 8 * h < rows_of(b)) {
+                const float* from = p.q + row_at(b, g + 8 * h) * HD + c;
+                q[h] = pack_bf16(from[0], from[1]);
+                q[2 + h] = pack_bf16(from[8], from[9]);
+            }
+        q_fragments[f * 32 + lane] = make_uint4(q[0], q[1], q[2], q[3]);
     }
-    const int most = warp_max_int(max(limit[0], limit[1]));                                          // keys that some row of the warp sees
-    const int all = -warp_max_int(-min(live[0] ? limit[0] : INT32_MAX, live[1] ? limit[1] : INT32_MAX));   // keys that every live row sees
-    const float scale2 = p.scale * 1.4426950408889634f;   // scores in units of log2 e: the weights are powers of two
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
-    float o[HD / 8][4];
+    int limit[kPrefillBlocks][2];   // keys that this thread's two rows of a block see
 #pragma unroll
-    for (int j = 0; j < HD / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
-
-    for (int i = 0; i < pages; ++i) {
-        const int s = i % S::stages;
-        if (threadIdx.x == 0 && i >= kLag && i - kLag + S::stages < pages) {
-            // (a wait that runs out leaves the page unrequested: everyone's wait for it runs out too)
-            if (mbar_wait(&empty[(i - kLag) % S::stages], ((i - kLag) / S::stages) & 1)) request(i - kLag + S::stages);
-            else atomicExch(p.status, B200_DEVICE_TIMEOUT);
+    for (int b = 0; b < kPrefillBlocks; ++b)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = g + 8 * h;
+            limit[b][h] = r < rows_of(b) ? base_len + (p.causal ? t_first + b * positions + r / group + 1 : 0) : 0;
         }
+    const int seen_by_all = base_len + (p.causal ? t_first + 1 : 0);   // keys that every row of the CTA sees
+    __syncthreads();
+
+    float m_row[kPrefillBlocks][2], l_row[kPrefillBlocks][2], o[kPrefillBlocks][HD / 8][4];
+#pragma unroll
+    for (int b = 0; b < kPrefillBlocks; ++b) {
+        m_row[b][0] = m_row[b][1] = -INFINITY;
+        l_row[b][0] = l_row[b][1] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < HD / 8; ++j) o[b][j][0] = o[b][j][1] = o[b][j][2] = o[b][j][3] = 0.0f;
+    }
+    const int tok0 = (warp & (kGroupWarps - 1)) * 16;
+    for (int i = warp / kGroupWarps; i < pages; i += kConsumerWarps / kGroupWarps) {
+        const int s = i % S::stages;
+        if (threadIdx.x == 0)
+            for (int j = i - kLag; j < i - kLag + 2; ++j) {   // (a wait that runs out leaves a page unrequested: everyone's wait for it runs out too)
+                if (j < 0 || j + S::stages >= pages) continue;
+                if (requested == j + S::stages && mbar_wait(&empty[j % S::stages], (j / S::stages) & 1)) request();
+            }
         __syncwarp();
         if (!mbar_wait(&full[s], (i / S::stages) & 1)) {
             if (lane == 0) atomicExch(p.status, B200_DEVICE_TIMEOUT);
+            *static_cast<volatile int*>(&gave_up) = 1;
             break;
         }
-        if (i * kFastPageSize < most) {
-            const uint32_t kbase = smem_u32(smem + s * S::stage_bytes), vbase = kbase + S::tile_bytes;
-            float sc[8][4];
+        const uint32_t kbase = smem_u32(smem + s * S::stage_bytes), vbase = kbase + S::tile_bytes;
+        float sc[kPrefillBlocks][2][4];
 #pragma unroll
-            for (int n = 0; n < 8; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.0f;
+        for (int b = 0; b < kPrefillBlocks; ++b)
 #pragma unroll
-            for (int kk = 0; kk < HD / 16; ++kk)
+            for (int n = 0; n < 2; ++n) sc[b][n][0] = sc[b][n][1] = sc[b][n][2] = sc[b][n][3] = 0.0f;
 #pragma unroll
-                for (int n = 0; n < 8; n += 2) {
-                    uint32_t r[4];
-                    ldmatrix_x4(r, kbase + tile_offset(n * 8 + (mi >> 1) * 8 + ri, 2 * kk + (mi & 1)));
-                    mma_bf16(sc[n], qa[kk], r[0], r[1]);
-                    mma_bf16(sc[n + 1], qa[kk], r[2], r[3]);
-                }
-            if ((i + 1) * kFastPageSize > all) {
+        for (int kk = 0; kk < HD / 16; ++kk) {
+            uint32_t r[4];
+            ldmatrix_x4(r, kbase + tile_offset(tok0 + (mi >> 1) * 8 + ri, 2 * kk + (mi & 1)));
 #pragma unroll
-                for (int n = 0; n < 8; ++n)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (i * kFastPageSize + n * 8 + 2 * t + (e & 1) >= limit[e >> 1]) sc[n][e] = -INFINITY;
+            for (int b = 0; b < kPrefillBlocks; ++b) {
+                const uint4 packed = q_fragments[(b * (HD / 16) + kk) * 32 + lane];
+                const uint32_t q[4] = {packed.x, packed.y, packed.z, packed.w};
+                mma_bf16(sc[b][0], q, r[0], r[1]);
+                mma_bf16(sc[b][1], q, r[2], r[3]);
             }
-            float base[2];
+        }
+        const bool masked = (i + 1) * kFastPageSize > seen_by_all;
+        const int token = i * kFastPageSize + tok0 + 2 * t;
+        uint32_t pa[kPrefillBlocks][4];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float high = fmaxf(sc[0][2 * h], sc[0][2 * h + 1]);
+        for (int b = 0; b < kPrefillBlocks; ++b) {
+            // scale, mask keys at or beyond the row's key count, online softmax per row (g and g + 8)
+            float mx[2] = {-INFINITY, -INFINITY}, corr[2], safe[2], sum[2] = {0.0f, 0.0f};
 #pragma unroll
-                for (int n = 1; n < 8; ++n) high = fmaxf(high, fmaxf(sc[n][2 * h], sc[n][2 * h + 1]));
-                high = fmaxf(high, __shfl_xor_sync(0xffffffffu, high, 1));
-                high = fmaxf(high, __shfl_xor_sync(0xffffffffu, high, 2));
-                const float next = fmaxf(m[h], high * scale2);
-                base[h] = next == -INFINITY ? 0.0f : next;
-                const float factor = exp2_fast(m[h] - base[h]);
-                m[h] = next;
-                l[h] *= factor;
-#pragma unroll
-                for (int j = 0; j < HD / 8; ++j) { o[j][2 * h] *= factor; o[j][2 * h + 1] *= factor; }
-            }
-#pragma unroll
-            for (int n = 0; n < 8; ++n)
+            for (int n = 0; n < 2; ++n)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    sc[n][e] = exp2_fast(fmaf(sc[n][e], scale2, -base[e >> 1]));
-                    l[e >> 1] += sc[n][e];
+                    float v = sc[b][n][e] * p.scale;
+                    if (masked && token + n * 8 + (e & 1) >= limit[b][e >> 1]) v = -INFINITY;
+                    sc[b][n][e] = v;
+                    mx[e >> 1] = fmaxf(mx[e >> 1], v);
                 }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t pa[4] = {pack_bf16(sc[2 * k][0], sc[2 * k][1]), pack_bf16(sc[2 * k][2], sc[2 * k][3]),
-                                        pack_bf16(sc[2 * k + 1][0], sc[2 * k + 1][1]), pack_bf16(sc[2 * k + 1][2], sc[2 * k + 1][3])};
+            for (int h = 0; h < 2; ++h) {
+                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+                const float m_new = fmaxf(m_row[b][h], mx[h]);
+                safe[h] = m_new == -INFINITY ? 0.0f : m_new;
+                corr[h] = expf(m_row[b][h] - safe[h]);
+                m_row[b][h] = m_new;
+            }
 #pragma unroll
-                for (int j = 0; j < HD / 8; j += 2) {
-                    uint32_t r[4];
-                    ldmatrix_x4_trans(r, vbase + tile_offset(k * 16 + (mi & 1) * 8 + ri, j + (mi >> 1)));
-                    mma_bf16(o[j], pa, r[0], r[1]);
-                    mma_bf16(o[j + 1], pa, r[2], r[3]);
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    sc[b][n][e] = expf(sc[b][n][e] - safe[e >> 1]);
+                    sum[e >> 1] += sc[b][n][e];
                 }
+            l_row[b][0] = l_row[b][0] * corr[0] + sum[0];
+            l_row[b][1] = l_row[b][1] * corr[1] + sum[1];
+#pragma unroll
+            for (int j = 0; j < HD / 8; ++j) {
+                o[b][j][0] *= corr[0]; o[b][j][1] *= corr[0];
+                o[b][j][2] *= corr[1]; o[b][j][3] *= corr[1];
+            }
+            pa[b][0] = pack_bf16(sc[b][0][0], sc[b][0][1]);
+            pa[b][1] = pack_bf16(sc[b][0][2], sc[b][0][3]);
+            pa[b][2] = pack_bf16(sc[b][1][0], sc[b][1][1]);
+            pa[b][3] = pack_bf16(sc[b][1][2], sc[b][1][3]);
+        }
+#pragma unroll
+        for (int j = 0; j < HD / 8; j += 2) {
+            uint32_t r[4];
+            ldmatrix_x4_trans(r, vbase + tile_offset(tok0 + (mi & 1) * 8 + ri, j + (mi >> 1)));
+#pragma unroll
+            for (int b = 0; b < kPrefillBlocks; ++b) {
+                mma_bf16(o[b][j], pa[b], r[0], r[1]);
+                mma_bf16(o[b][j + 1], pa[b], r[2], r[3]);
             }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
     }
+    __syncthreads();   // every page has been consumed: the stages can be reused for the merge
+    if (gave_up) {     // ... unless a wait ran out: pages that are on their way get the same time again before the CTA leaves
+        if (threadIdx.x == 0)
+            for (int j = max(0, requested - S::stages); j < requested; ++j) mbar_wait(&full[j % S::stages], (j / S::stages) & 1);
+        __syncthreads();
+        return;
+    }
+
+    float* merge_o = reinterpret_cast<float*>(smem);                     // [blocks][warps][16][pitch]
+    float* merge_ml = merge_o + S::units * S::pitch;                       // [blocks][warps][16][2]
+    float* weights = merge_ml + S::units * 2;                              // [blocks][16][warps]
+    float* sums = weights + S::units;                                      // [blocks][16]
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
-        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
-        if (!live[h] || limit[h] == 0) continue;   // (a row that sees no key is left as it is)
-        const int64_t at = (static_cast<int64_t>(at_row[h]) * p.heads + at_head[h]) * HD + 2 * t;
+    for (int b = 0; b < kPrefillBlocks; ++b)
 #pragma unroll
-        for (int j = 0; j < HD / 8; ++j) {
-            const float a = o[j][2 * h] / l[h], b = o[j][2 * h + 1] / l[h];
-            if (p.out_hi) {
-                const __nv_bfloat162 hi = __floats2bfloat162_rn(a, b);
-                *reinterpret_cast<__nv_bfloat162*>(p.out_hi + at + j * 8) = hi;
-                *reinterpret_cast<__nv_bfloat162*>(p.out_lo + at + j * 8) = __floats2bfloat162_rn(a - __low2float(hi), b - __high2float(hi));
-            } else {
-                *reinterpret_cast<float2*>(p.out + at + j * 8) = make_float2(a, b);
+        for (int h = 0; h < 2; ++h) {
+            float l = l_row[b][h];
+            l += __shfl_xor_sync(0xffffffffu, l, 1);
+            l += __shfl_xor_sync(0xffffffffu, l, 2);
+            const int unit = (b * kConsumerWarps + warp) * 16 + g + 8 * h;
+            float* to = merge_o + unit * S::pitch + 2 * t;
+#pragma unroll
+            for (int j = 0; j < HD / 8; ++j) *reinterpret_cast<float2*>(to + j * 8) = make_float2(o[b][j][2 * h], o[b][j][2 * h + 1]);
+            if (t == 0) {
+                merge_ml[2 * unit] = m_row[b][h];
+                merge_ml[2 * unit + 1] = l;
             }
         }
+    __syncthreads();
+    {   // eight adjacent lanes are the eight warps' parts of one row
+        static_assert(S::units == kPrefillThreads);
+        const int row = threadIdx.x >> 3, w = threadIdx.x & 7, unit = ((row >> 4) * kConsumerWarps + w) * 16 + (row & 15);
+        const float mw = merge_ml[2 * unit], lw = merge_ml[2 * unit + 1];
+        float m = mw;
+#pragma unroll
+        for (int x = 1; x < 8; x <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, x));
+        const float weight = mw == -INFINITY ? 0.0f : expf(mw - m);
+        float l = 0.0f;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) l += __shfl_sync(0xffffffffu, weight, (lane & 24) + x) * __shfl_sync(0xffffffffu, lw, (lane & 24) + x);
+        weights[threadIdx.x] = weight;
+        if (w == 0) sums[row] = l;
     }
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < kPrefillBlocks; ++b)
+        for (int i = threadIdx.x; i < rows_of(b) * HD; i += kPrefillThreads) {
+            const int r = i / HD, d = i - r * HD;
+            const float* part = merge_o + (b * kConsumerWarps * 16 + r) * S::pitch + d;
+            const float* weight = weights + (b * 16 + r) * kConsumerWarps;
+            float acc = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kConsumerWarps; ++w) acc += weight[w] * part[w * 16 * S::pitch];
+            store_result(p, row_at(b, r) * HD + d, acc / sums[b * 16 + r]);
+        }
 }
 
 // Generic path: one (row, head) per CTA, eight warps that take kGenericTokens tokens of the split at a time.  Bound by latency (the f32 byte
@@ -966,23 +1039,28 @@ __global__ void attention_combine_kernel(const AttnParams p) {
     }
 }
 
-// Whether a pass takes the prefill kernel: at least three of its eight warps have rows (below that, attention_mma_kernel's warps, which share
-// out a page's tokens, stream the cache faster), and either the context is short (a page costs a CTA here 1.0 us in a chain, there 0.4, but
-// the fixed part is 4 us against 6) or that kernel's CTAs need more than one round.  us, this | attention_mma_kernel: 1 sequence, 12 positions
-// behind 1000: 19.6 | 12.0; 32 of them: 25.6 | 44.9; 64 x 16 positions from the start: 6.0 | 26.0; heads of 128, 8 x 12 behind 500: 15.8 | 24.0.
-constexpr int kPrefillFrom = 48, kPrefillShort = 6;
-bool takes_prefill(int tokens, int group, int64_t items, int pages, int head_dim, int sms) {
-    return tokens * static_cast<int64_t>(group) >= kPrefillFrom && (pages <= kPrefillShort || items > (head_dim == 64 ? 2 : 1) * sms);
+// Whether a pass takes the prefill kernel: where its half as many CTAs save rounds over the SMs.  A round costs about 8 + pages us there, 8 +
+// 0.53 pages with attention_mma_kernel (the results are the same); CTAs with heads of 64, two per SM, gain little from having an SM to
+// themselves.  us, attention_mma_kernel | prefill kernel: 48 positions behind 1000, heads of 64, 1 sequence 12.6 | 18.0, 4 sequences 26.9 | 24.2,
+// 16 83.8 | 67.4; 100 positions behind 4000, heads of 128, 1 sequence 80 | 69, 200 positions 120 | 138.  Over 180 sizes up to 13 % from the better one.
+bool takes_prefill(int64_t items, int64_t ctas, int pages, int head_dim, int sms) {
+    auto rounds = [&](int64_t n) {
+        const double whole = static_cast<double>((n + sms - 1) / sms);
+        return head_dim == 64 && whole < 1.45 ? 1.45 : whole;
+    };
+    return rounds(ctas) * (8.0 + pages) < rounds(items) * (8.0 + 0.53 * pages);
 }
 
-template <int HD> int launch_prefill(const b200_kv_cache* cache, AttnParams p, cudaStream_t stream) {
-    using S = FastShape<HD, prefill_stages<HD>()>;
-    p.positions_per_item = kPrefillRows / (p.heads / p.kv.kv_heads);
-    const int64_t ctas = static_cast<int64_t>(p.kv.sequences) * p.kv.kv_heads * ((p.tokens_per_sequence + p.positions_per_item - 1) / p.positions_per_item);
+int64_t prefill_ctas(const AttnParams& p) {
+    const int span = kPrefillBlocks * p.positions_per_item;
+    return static_cast<int64_t>(p.kv.sequences) * p.kv.kv_heads * ((p.tokens_per_sequence + span - 1) / span);
+}
+
+template <int HD> int launch_prefill(const b200_kv_cache* cache, const AttnParams& p, cudaStream_t stream) {
     auto kernel = attention_prefill_kernel<HD>;
-    B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::smem_bytes));
-    return cuda_status(launch_dependent(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kPrefillThreads), S::smem_bytes, stream, *kv_tensor_map(cache, 0),
-                                        *kv_tensor_map(cache, 1), p), "attention_prefill_kernel launch");
+    B200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PrefillShape<HD>::smem_bytes));
+    return cuda_status(launch_dependent(kernel, dim3(static_cast<unsigned>(prefill_ctas(p))), dim3(kPrefillThreads), PrefillShape<HD>::smem_bytes, stream,
+                                        *kv_tensor_map(cache, 0), *kv_tensor_map(cache, 1), p), "attention_prefill_kernel launch");
 }
 
 // Clusters of `splits` CTAs that the device holds at once; asked of the runtime once per device and size, and kept.
@@ -1130,9 +1208,7 @@ int attention_launch(const float* q, int64_t rows, int32_t tokens_per_sequence, 
         // drain overlap the other's streaming; with fewer CTAs each keeps the deeper ring to itself.
         const int64_t ctas = (static_cast<int64_t>(p.rows) / tokens_per_sequence) * ((tokens_per_sequence + positions - 1) / positions)
                              * p.kv.kv_heads * p.num_splits;
-        // pairs of results are stored together: the planes and rows that callers hand in are 4- and 8-byte aligned for that
-        const bool pairs = ((out_hi ? (reinterpret_cast<uintptr_t>(out_hi) | reinterpret_cast<uintptr_t>(out_lo)) << 1 : reinterpret_cast<uintptr_t>(out)) & 7) == 0;
-        if (tokens_per_sequence > 1 && pairs && takes_prefill(tokens_per_sequence, group, ctas, plan.pages_total, cache->head_dim, sm_count(device)))
+        if (tokens_per_sequence > 1 && takes_prefill(ctas, prefill_ctas(p), plan.pages_total, cache->head_dim, sm_count(device)))
             return cache->head_dim == 128 ? launch_prefill<128>(cache, p, s) : launch_prefill<64>(cache, p, s);
         if (cache->head_dim == 128) status = launch_fast<128, 6>(cache, p, merged, s);
         else if (ctas > sm_count(device)) status = launch_fast<64, 6>(cache, p, merged, s);

@@ -330,15 +330,15 @@ def test_chunk_attention_is_causal(cache_dtype, hd):
 
 
 @pytest.mark.parametrize("hd,heads,kv_heads,n,prefix,L,causal", [
-    (64, 8, 2, 2, 0, 193, 1),      # blocks of 32 positions x 4 heads, the last one short
-    (64, 12, 4, 1, 70, 101, 1),    # a group of three: 42 positions and two rows to spare; starts inside a page
-    (128, 16, 16, 1, 5, 300, 1),   # one head per cached head: 128 positions a block
-    (128, 16, 4, 10, 640, 40, 1),  # more pages than ring stages: taken for its 400 items
-    (128, 16, 1, 2, 300, 9, 1),    # a group of 16
-    (64, 16, 1, 20, 2300, 20, 1),  # a group of 16 behind a context that the other kernels would split
-    (64, 4, 1, 1, 300, 12, 1),     # exactly the rows from which the kernel is taken
-    (64, 4, 1, 1, 500, 12, 1),     # a longer context of few items: the token-split kernel
-    (64, 8, 2, 3, 130, 33, 0),     # not causal: every row sees the prefix
+    (64, 8, 2, 9, 0, 193, 1),      # pairs of blocks of 4 positions x 4 heads, the last one short
+    (64, 12, 4, 10, 70, 101, 1),   # a group of three: 5 positions and a row to spare; starts inside a page
+    (128, 16, 16, 5, 5, 300, 1),   # one head per cached head: 16 positions a block
+    (128, 16, 4, 10, 640, 40, 1),  # more pages than ring stages
+    (128, 16, 1, 20, 300, 9, 1),   # a group of 16: a position a block, the last pair half empty
+    (64, 16, 1, 30, 2300, 20, 1),  # a group of 16 behind a context that the other kernels would split
+    (64, 4, 1, 1, 300, 12, 1),     # few items: a block per CTA
+    (64, 4, 1, 1, 500, 12, 1),
+    (64, 8, 2, 30, 130, 33, 0),    # not causal: every row sees the prefix
 ])
 def test_prefill_attention_blocks(hd, heads, kv_heads, n, prefix, L, causal):
     """Many positions per sequence on unequal block, page and ring borders (bf16 cache; bf16 queries and weights: the tolerance of the others)."""
@@ -356,6 +356,24 @@ def test_prefill_attention_blocks(hd, heads, kv_heads, n, prefix, L, causal):
     sees = torch.arange(cap)[None] < (torch.arange(L)[:, None] + prefix + 1 if causal else prefix)
     want = (score.masked_fill(~sees, -np.inf).softmax(-1) @ v).transpose(1, 2).numpy()
     assert rel(got, want) < 1e-2
+
+
+@pytest.mark.parametrize("hd,heads,kv_heads,n,prefix,L,causal", [
+    (64, 12, 4, 8, 70, 101, 1), (64, 8, 2, 8, 0, 193, 1), (64, 16, 1, 40, 500, 9, 1), (64, 4, 4, 36, 600, 33, 1), (128, 8, 2, 8, 290, 40, 1),
+    (128, 16, 16, 8, 5, 130, 1), (64, 8, 2, 40, 130, 33, 0)])
+def test_prefill_attention_is_that_of_single_positions(hd, heads, kv_heads, n, prefix, L, causal):
+    """A row's result does not hang on how many positions a pass has: bit for bit what a call for this position alone gives (calls of at most 148
+    items: beyond, a persistent CTA deals its pages to the warps across items)."""
+    rng = np.random.default_rng(hd + heads + L)
+    cap = prefix + L
+    cache = Cache(B.BF16, n, kv_heads, hd, cap)
+    cache.append(*(rng.standard_normal((n, kv_heads, cap, hd), dtype=np.float32) for _ in range(2)))
+    cache.set_lengths(np.full(n, prefix, dtype=np.int32))
+    q = rng.standard_normal((n, L, heads, hd), dtype=np.float32)
+    together = attention(q.reshape(n * L, heads, hd), cache, L, heads, cap, causal).reshape(n, L, -1)
+    for t in sorted({0, 1, L // 2, L - 1}):
+        cache.set_lengths(np.full(n, prefix + (t if causal else 0), dtype=np.int32))
+        assert np.array_equal(together[:, t], attention(q[:, t], cache, 1, heads, cap, causal)), t
 
 
 def test_attention_linearity_in_values_at_long_context():
