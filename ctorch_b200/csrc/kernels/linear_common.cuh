@@ -225,7 +225,7 @@ bool linear_stream_takes(int rows, int in);   // a shadow call with these sizes 
 int linear_argmax_parts(int rows, int in, int out);
 // tcgen05 GEMM for many rows (linear_gemm.cu): shadow input only; B200_UNSUPPORTED otherwise.
 int launch_linear_gemm(const LinearParams& p, int epilogue, cudaStream_t stream);
-int linear_gemm_parts(int rows, int in, int out);
+int linear_gemm_parts(int rows, int in, int out, bool residual);   // (residual: partial sums of squares; else slices of the greedy choice)
 // Row count from which the dense tensor-core kernel replaces the streaming one.
 constexpr int kGemmRows = 17;
 // Decode batches on the tensor cores with the weights as the streamed operand (linear_decode.cu): up to 256 rows.

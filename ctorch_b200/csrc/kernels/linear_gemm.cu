@@ -543,8 +543,6 @@ int encode_operand(CUtensorMap* map, const void* base, int rows, int columns, in
     return B200_OK;
 }
 
-// Tile width of a launch: 128 features; 256 only for very wide matrices (vocabulary projections), where the tiles still
-// fill the SMs several times over and the wide tile halves the activation bytes pulled per weight byte.
 // Launches the persistent kernel serves: prefill-sized passes (8 or more token tiles, more tiles than SMs) whose K is short
 // enough that the epilogues are a large share of a tile's time (measured: K 768 +28 %, K 2048 +5 %, K 8192 -11 % against the
 // one-tile-per-CTA kernel with the wide tile).
@@ -573,12 +571,23 @@ bool wide_operands(const LinearParams& p, int epilogue) {
     return false;
 }
 
+// Tile width of the other kernels' launches: 128 features; 256 where the tiles still fill the SMs several times over, since the wide tile halves
+// the activation bytes pulled per weight byte (greedy choices of long passes beyond K = 2048, operands that the wide kernel refuses).
 int choose_tile_features(int rows, int in, int out) {
     int device = 0, sms = 148;
     if (cudaGetDevice(&device) == cudaSuccess) sms = sm_count(device);
-    if (takes_persistent(rows, in, out, sms) || takes_wide(rows, out, sms)) return 128;   // (the wide kernel leaves a partial per 128 features)
+    if (takes_persistent(rows, in, out, sms)) return 128;
     const int row_tiles = (rows + kTileM - 1) / kTileM;
     return row_tiles * ((out + 255) / 256) >= 2 * sms ? 256 : 128;
+}
+
+// The same where a call has the wide kernel's sizes and an epilogue of two kinds.  Residual: partial sums of squares are counted from the sizes alone;
+// the wide kernel leaves one per 128 features, and so does what serves operands that it refuses.  q|k|v with adapters: their deltas outweigh
+// what wider tiles save (1600 | 2048 | 8192 rows of 4096 -> 6144, rank 16: 203 | 218 | 876 us with 128 features, 212 | 232 | 867 with 256).
+int narrow_tile_features(int rows, int in, int out) {
+    int device = 0, sms = 148;
+    if (cudaGetDevice(&device) == cudaSuccess) sms = sm_count(device);
+    return takes_wide(rows, out, sms) ? 128 : choose_tile_features(rows, in, out);
 }
 
 // Ring depth for the 128-wide tile: two stages (96 KB) let two CTAs share an SM, so one tile's epilogue and pipeline ramp overlap the other's
@@ -628,9 +637,9 @@ int launch_epilogue(int epilogue, const CUtensorMap& hi, const CUtensorMap& lo, 
 
 }  // namespace
 
-int linear_gemm_parts(int rows, int in, int out) {
+int linear_gemm_parts(int rows, int in, int out, bool residual) {
     if (linear_decode_takes(rows)) return linear_decode_parts(rows, in, out);
-    const int tn = choose_tile_features(rows, in, out);
+    const int tn = residual ? narrow_tile_features(rows, in, out) : choose_tile_features(rows, in, out);
     return (out + tn - 1) / tn;   // one partial per feature tile: a row of a tile is finished by one CTA of the cluster
 }
 
@@ -697,7 +706,8 @@ int launch_linear_gemm(const LinearParams& p, int epilogue, cudaStream_t stream)
         return status != B200_OK ? status : launch_wide(epilogue, hi, lo, w, gp, sms, stream);
     }
     const bool persistent = takes_persistent(p.rows, p.in, p.out, sms);
-    const int tn = persistent ? 128 : choose_tile_features(p.rows, p.in, p.out);
+    const bool narrow = epilogue == B200_EPI_RESIDUAL || (epilogue == B200_EPI_QKV && p.lora_rank > 0);
+    const int tn = narrow ? narrow_tile_features(p.rows, p.in, p.out) : choose_tile_features(p.rows, p.in, p.out);
     int status = encode_operand(&hi, p.x_hi, p.rows, p.in, kTileM);
     if (status == B200_OK) status = encode_operand(&lo, p.x_lo ? p.x_lo : p.x_hi, p.rows, p.in, kTileM);
     if (status == B200_OK) status = encode_operand(&w, p.weight, p.out, p.in, tn);

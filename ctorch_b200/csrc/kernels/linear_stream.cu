@@ -585,12 +585,12 @@ bool linear_stream_takes(int rows, int in) { return rows < kGemmRows && (in <= k
 
 int linear_stream_parts(int rows, int in, int out) {
     if ((in & 7) || in <= 0 || out <= 0) return 0;
-    return linear_stream_takes(rows, in) ? (out + kFewFeatures - 1) / kFewFeatures : linear_gemm_parts(rows, in, out);
+    return linear_stream_takes(rows, in) ? (out + kFewFeatures - 1) / kFewFeatures : linear_gemm_parts(rows, in, out, true);
 }
 
 int linear_argmax_parts(int rows, int in, int out) {
     if ((in & 7) || in <= 0 || out <= 0) return 0;
-    if (!linear_stream_takes(rows, in)) return linear_gemm_parts(rows, in, out);
+    if (!linear_stream_takes(rows, in)) return linear_gemm_parts(rows, in, out, false);
     int device = -1;
     if (cudaGetDevice(&device) != cudaSuccess) { cudaGetLastError(); device = -1; }   // no device: the figures of a 148-SM part
     return few_groups(in, out, sm_count(device)).total();   // one candidate slice per group

@@ -676,6 +676,39 @@ def test_wide_linear_appends_q_k_v(cache_dtype, heads, kv_heads, hd):
         assert rel(cache.gather(1, end)[b][:, lengths[b]:end], y[b, :, D + KV:].reshape(L, kv_heads, hd).transpose(1, 0, 2)) < tol
 
 
+@pytest.mark.parametrize("n,L,inner,rank", [(5, 1, 256, 8), (32, 1, 256, 8), (40, 1, 512, 24), (20, 1, 256, 4), (4, 50, 256, 24),   # decode kernels
+                                            (8, 150, 256, 8), (8, 150, 2304, 24)])                      # long passes: short K, tiles of 256 features
+def test_adapters_of_the_q_k_v_epilogue(n, L, inner, rank):
+    """Adapter deltas of q and v, ranks that end a batch of 16 halfway and that are no multiple of eight; f32 cache, so that nothing is rounded."""
+    l = B.lib()
+    heads, kv_heads, hd, cap = 16, 4, 128, 230
+    D, KV, scale = heads * hd, kv_heads * hd, 0.5
+    g = torch.Generator(device="cuda").manual_seed(inner + rank)
+    normal = lambda *shape: torch.randn(shape, generator=g, device="cuda")
+    x = normal(n * L, inner)
+    hi = x.bfloat16()
+    lo = (x - hi.float()).bfloat16()
+    w = (normal(D + 2 * KV, inner) * inner ** -0.5).bfloat16()
+    low, q_up, v_up = normal(n * L, 2 * rank), normal(D, rank).bfloat16(), normal(KV, rank).bfloat16()
+    still = torch.ones((cap, hd // 2), device="cuda"), torch.zeros((cap, hd // 2), device="cuda")   # (rotations have their own test)
+    cache = Cache(B.F32, n, kv_heads, hd, cap)
+    cache.set_lengths(np.full(n, 3, dtype=np.int32))
+    q = torch.full((n * L, D), float("nan"), device="cuda")
+    qkv = B.QkvArgs(heads, kv_heads, hd, L, still[0].data_ptr(), still[1].data_ptr(), cap, cache.h.value, q.data_ptr(), rank, scale, low.data_ptr(),
+                    q_up.data_ptr(), v_up.data_ptr())
+    args = B.ShadowLinearArgs(x_hi=hi.data_ptr(), x_lo=lo.data_ptr(), rows=n * L, inner=inner, weight=w.data_ptr(), out=D + 2 * KV, epilogue=3, qkv=C.pointer(qkv))
+    torch.cuda.synchronize()
+    B.kcheck(l.b200_linear_shadow(C.byref(args), stream()))
+    sync()
+    y = (hi.double() + lo.double()) @ w.double().T
+    y[:, :D] += scale * low[:, :rank].double() @ q_up.double().T
+    y[:, D + KV:] += scale * low[:, rank:].double() @ v_up.double().T
+    y = y.cpu().numpy()
+    assert rel(q.cpu().numpy(), y[:, :D]) < 3e-5
+    for which, part in ((0, y[:, D:D + KV]), (1, y[:, D + KV:])):
+        assert rel(cache.gather(which, 3 + L)[:, :, 3:], part.reshape(n, L, kv_heads, hd).transpose(0, 2, 1, 3)) < 3e-5
+
+
 @pytest.mark.parametrize("rows,inner,vocab", [(16, 768, 32000), (5, 256, 1000), (40, 512, 5000), (32, 2048, 1024), (200, 256, 777 * 2),
                                               (20, 256, 76000)])
 def test_fused_logits_argmax(rows, inner, vocab):

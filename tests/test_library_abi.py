@@ -135,6 +135,15 @@ def test_shadow_linear_dispatch_by_row_count():
     assert name(32, 4096, 32) == "linear_thin_kernel"
 
 
+def test_tiles_of_long_passes_follow_the_epilogue():
+    """Beyond K = 2048 the kernel with the register epilogue leaves a partial sum per 128 features; greedy choices are not its work and have the tiles
+    of 256 features."""
+    l = B.lib()
+    assert l.b200_linear_shadow_parts(2048, 4096, 16384) == 128 and l.b200_linear_argmax_parts(2048, 4096, 16384) == 64
+    assert l.b200_linear_shadow_parts(2048, 2048, 16384) == l.b200_linear_argmax_parts(2048, 2048, 16384) == 128
+    assert l.b200_linear_argmax_parts(1024, 4096, 4096) == 32   # too few tiles for the wider ones
+
+
 def test_decode_launch_shapes_fit_the_sm():
     """The cost-model search of the decode-batch kernel, on the host: for the projection sizes of every BASELINE
     configuration and some odd ones, at every row count it serves, the shape it picks fits an SM (227 KB of shared memory,
