@@ -321,9 +321,10 @@ __global__ void __launch_bounds__(kFinishWarps * 32) argmax_finish_kernel(const 
     __syncthreads();
     if (!last) return;
     // end of a step: the caches (one per layer) move on by the token every earlier kernel of the step appended and read
-    // (a warp per cache: one after the other, the caches' round trips to L2 took 8 of the launch's 11.5 us at 16 layers)
+    // (a warp per cache: one after the other, the caches' round trips to L2 took 8 of the launch's 11.5 us at 16 layers; atomic, since a list may
+    // name a cache twice, which then moves on by two)
     for (int c = warp; c < advance.caches; c += kFinishWarps)
-        for (int i = lane; i < advance.counts[c]; i += 32) advance.lengths[c][i] += 1;
+        for (int i = lane; i < advance.counts[c]; i += 32) atomicAdd(advance.lengths[c] + i, 1);
     __syncthreads();
     if (threadIdx.x == 0) {
         argmax_finish_ticket = 0;

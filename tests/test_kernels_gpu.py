@@ -709,6 +709,29 @@ def test_adapters_of_the_q_k_v_epilogue(n, L, inner, rank):
         assert rel(cache.gather(which, 3 + L)[:, :, 3:], part.reshape(n, L, kv_heads, hd).transpose(0, 2, 1, 3)) < 3e-5
 
 
+class DeviceInts:
+    def __init__(self, pointer, count):
+        self.__cuda_array_interface__ = {"shape": (count,), "typestr": "<i4", "data": (pointer, False), "version": 3}
+
+
+def test_a_cache_named_again_moves_on_again():
+    """Lengths at the end of a step, a warp per cache: 70 sequences, more caches than warps, one of them named three times, by several warps."""
+    l = B.lib()
+    caches = [Cache(B.F32, 70, 1, 16, 64) for _ in range(9)]
+    for c in caches:
+        c.set_lengths(np.arange(70, dtype=np.int32) % 50)
+    named = [caches[i] for i in (0, 1, 0, 2, 3, 4, 5, 6, 7, 8, 0)]
+    value, index = torch.zeros((1, 3), device="cuda"), torch.zeros((1, 3), dtype=torch.int32, device="cuda")
+    next_ids, counter = torch.zeros(3, dtype=torch.int64, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    B.kcheck(l.b200_argmax_finish(value.data_ptr(), index.data_ptr(), 1, 3, next_ids.data_ptr(), None, None, 0, counter.data_ptr(),
+                                  (C.c_void_p * len(named))(*(c.h for c in named)), len(named), stream()))
+    sync()
+    for i, c in enumerate(caches):
+        got = torch.as_tensor(DeviceInts(l.b200_kv_cache_lengths(c.h), 70), device="cuda").cpu().numpy()
+        assert np.array_equal(got, np.arange(70) % 50 + (3 if i == 0 else 1))
+
+
 @pytest.mark.parametrize("rows,inner,vocab", [(16, 768, 32000), (5, 256, 1000), (40, 512, 5000), (32, 2048, 1024), (200, 256, 777 * 2),
                                               (20, 256, 76000)])
 def test_fused_logits_argmax(rows, inner, vocab):
