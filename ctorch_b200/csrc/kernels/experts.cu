@@ -550,6 +550,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_gemm_wide_kernel(const
     constexpr uint32_t kWhole = mma_instruction_bf16(kTile, kWideN), kHalf = mma_instruction_bf16(kTile, kTile);
     const LinearParams& p = gp.base;
     extern __shared__ uint8_t smem_raw[];
+    __shared__ WideFlight flight;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kWideStages * kWideStageBytes);
     uint64_t* empty = full + kWideStages;
@@ -567,6 +568,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_gemm_wide_kernel(const
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 8);
         }
+        flight = {0, 0, 0};
         mbar_fence_init();
         tma_prefetch_descriptor(&map_hi);
         tma_prefetch_descriptor(&map_lo);
@@ -616,7 +618,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_gemm_wide_kernel(const
             for (int i = 0; i < k_blocks; ++i, ++it) {
                 const int s = it % kWideStages;
                 if (!mbar_wait(&empty[s], ((it / kWideStages) & 1) ^ 1)) {
-                    if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                    if (lane == 0) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); flight.gave_up = 1; }
                     alive = false;
                     break;
                 }
@@ -631,6 +633,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_gemm_wide_kernel(const
                 __syncwarp();
             }
         }
+        if (lane == 0) flight.loads = max(it, ahead);
     } else if (warp == 1) {
         int it = 0, j = 0;
         bool alive = true;
@@ -640,14 +643,14 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_gemm_wide_kernel(const
             const uint32_t instruction = width == kWideN ? kWhole : kHalf, accumulator = tmem_base + static_cast<uint32_t>((j & 1) * kWideN);
             // the epilogue of the tile that used this buffer two tiles ago must have read it (passes at once for j < 2)
             if (!mbar_wait(&acc_empty[j & 1], ((j >> 1) & 1) ^ 1)) {
-                if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                if (lane == 0) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); flight.gave_up = 1; }
                 break;
             }
             tc_fence_after_sync();
             for (int i = 0; i < k_blocks; ++i, ++it) {
                 const int s = it % kWideStages;
                 if (!mbar_wait(&full[s], (it / kWideStages) & 1)) {
-                    if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                    if (lane == 0) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); flight.gave_up = 1; }
                     alive = false;
                     break;
                 }
@@ -667,6 +670,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_gemm_wide_kernel(const
                 __syncwarp();
             }
         }
+        if (lane == 0) flight.products = it;
     } else {
         // ---- epilogue warps 2-9: TMEM lanes 32 * (warp % 4) .. + 31, features [128 * half, + 128) of the tile ----
         const int quarter = warp & 3, half = (warp - 2) >> 2, tile_row = quarter * 32 + lane;
@@ -678,7 +682,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_gemm_wide_kernel(const
             const int slot = tile_row < group.z ? group.y + tile_row : p.rows;   // rows past the group's hold no results
             const float scale = gp.scale && tile_row < group.z ? __ldg(gp.scale + slot) : 1.0f;
             if (!mbar_wait_relaxed(&acc_full[j & 1], (j >> 1) & 1)) {
-                if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                if (lane == 0) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); flight.gave_up = 1; }
                 break;
             }
             tc_fence_after_sync();
@@ -696,6 +700,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_gemm_wide_kernel(const
     __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
+    if (flight.gave_up) {
+        if (threadIdx.x == 0) wide_drain(flight, full, empty, kWideStages);
+        __syncthreads();
+    }
     if (warp == 1) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 2 * kWideN);

@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_gemm_wide_kernel(const
     constexpr uint32_t kWhole = mma_instruction_bf16(kTileM, kWideN), kHalf = mma_instruction_bf16(kTileM, 128);
     const LinearParams& p = gp.base;
     extern __shared__ uint8_t smem_raw[];
+    __shared__ WideFlight flight;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + kWideStages * kWideStageBytes);
     uint64_t* empty = full + kWideStages;
@@ -419,6 +420,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_gemm_wide_kernel(const
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 8);
         }
+        flight = {0, 0, 0};
         mbar_fence_init();
         tma_prefetch_descriptor(&map_hi);
         tma_prefetch_descriptor(&map_lo);
@@ -446,7 +448,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_gemm_wide_kernel(const
                 const uint32_t bytes = (has_lo ? 2 * kBoxBytes : kBoxBytes) + (width == kWideN ? 2 * kBoxBytes : kBoxBytes);
                 for (int i = 0; i < k_blocks; ++i, ++it) {
                     const int s = it % kWideStages;
-                    if (!mbar_wait(&empty[s], ((it / kWideStages) & 1) ^ 1)) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); alive = false; break; }
+                    if (!mbar_wait(&empty[s], ((it / kWideStages) & 1) ^ 1)) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); flight.gave_up = 1; alive = false; break; }
                     uint8_t* stage = smem + s * kWideStageBytes;
                     mbar_expect_tx(&full[s], bytes);
                     tma_load_2d(stage, &map_hi, i * kBlockK, m0, &full[s]);
@@ -455,6 +457,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_gemm_wide_kernel(const
                     if (width == kWideN) tma_load_2d(stage + 3 * kBoxBytes, &map_w, i * kBlockK, n0 + 128, &full[s]);
                 }
             }
+            flight.loads = it;
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -465,11 +468,11 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_gemm_wide_kernel(const
                 wide_place(plan, unit, p.out, m0, n0, width);
                 const uint32_t instruction = width == kWideN ? kWhole : kHalf, accumulator = tmem_base + static_cast<uint32_t>((j & 1) * kWideN);
                 // the epilogue of the tile that used this buffer two tiles ago must have read it (passes at once for j < 2)
-                if (!mbar_wait(&acc_empty[j & 1], ((j >> 1) & 1) ^ 1)) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); break; }
+                if (!mbar_wait(&acc_empty[j & 1], ((j >> 1) & 1) ^ 1)) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); flight.gave_up = 1; break; }
                 tc_fence_after_sync();
                 for (int i = 0; i < k_blocks; ++i, ++it) {
                     const int s = it % kWideStages;
-                    if (!mbar_wait(&full[s], (it / kWideStages) & 1)) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); alive = false; break; }
+                    if (!mbar_wait(&full[s], (it / kWideStages) & 1)) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); flight.gave_up = 1; alive = false; break; }
                     tc_fence_after_sync();
                     const uint32_t stage = smem_u32(smem + s * kWideStageBytes);
                     const uint64_t hi = operand_descriptor(stage), lo = operand_descriptor(stage + kBoxBytes), w = operand_descriptor(stage + 2 * kBoxBytes);
@@ -482,6 +485,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_gemm_wide_kernel(const
                 }
                 if (alive) tc_commit(&acc_full[j & 1]);
             }
+            flight.products = it;
         }
     } else {
         // ---- epilogue warps 2-9: TMEM lanes 32 * (warp % 4) .. + 31, features [128 * half, + 128) of the tile ----
@@ -502,7 +506,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_gemm_wide_kernel(const
             }
             if constexpr (EPI == B200_EPI_QKV) place = qkv_row_place(p, row);
             if (!mbar_wait_relaxed(&acc_full[j & 1], (j >> 1) & 1)) {
-                if (lane == 0) atomicExch(gp.status, B200_DEVICE_TIMEOUT);
+                if (lane == 0) { atomicExch(gp.status, B200_DEVICE_TIMEOUT); flight.gave_up = 1; }
                 break;
             }
             tc_fence_after_sync();
@@ -523,6 +527,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) linear_gemm_wide_kernel(const
     __syncwarp();
     tc_fence_before_sync();
     __syncthreads();
+    if (flight.gave_up) {
+        if (threadIdx.x == 0) wide_drain(flight, full, empty, kWideStages);
+        __syncthreads();
+    }
     if (warp == 1) {
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, 2 * kWideN);

@@ -8,6 +8,14 @@ namespace b200 {
 
 constexpr int kWideN = 256, kWideThreads = 320;   // features of a tile; producer warp, issuing warp, two epilogue warps per lane quarter
 
+// What a CTA has under way: K blocks requested and multiplied, and whether a bounded wait ran out.
+struct WideFlight { int loads, products, gave_up; };
+// After a wait that ran out, before the CTA leaves: copies and products that are under way get the same time again (one thread).
+__device__ __forceinline__ void wide_drain(const WideFlight& flight, uint64_t* full, uint64_t* empty, int stages) {
+    for (int j = max(0, flight.loads - stages); j < flight.loads; ++j) mbar_wait(&full[j % stages], (j / stages) & 1);
+    for (int j = max(0, flight.products - stages); j < flight.products; ++j) mbar_wait(&empty[j % stages], (j / stages) & 1);
+}
+
 __device__ __forceinline__ void pack_eight(const float* v, uint4& hi, uint4& lo) {
     uint32_t h[4], l[4];
 #pragma unroll
