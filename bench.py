@@ -620,7 +620,7 @@ def run_linear(args) -> dict:
                 {"bound": "tensor", "achieved": flops / seconds / 1e12, "peak": tensor_peak, "unit": "TFLOP/s", "peak_kind": "measured burst",
                  "algorithmic_flops": flops, "note": "useful flops; the kernel issues twice as many (activation hi + lo planes)"})
     roofline.update(frac=roofline["achieved"] / roofline["peak"], traffic=None,
-                    kernel="linear_stream_kernel" if rows <= 16 and inner <= 2048 else "linear_gemm_kernel", launch_ms=ms / args.steps)
+                    kernel=B.lib().b200_linear_shadow_kernel(rows, inner, out).decode(), launch_ms=ms / args.steps)
     line = {"metric": "linear_rows_per_s", "value": world * rows / seconds, "unit": "rows/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "bf16 weights, f32 activations as bf16 hi+lo, f32 accumulate", "data": "synthetic",

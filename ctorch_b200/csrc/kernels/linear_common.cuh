@@ -221,6 +221,7 @@ int launch_linear_stream(const LinearParams& p, int epilogue, cudaStream_t strea
 // Number of per-row sum-of-squares partials a residual-epilogue shadow call with these sizes writes (0: unsupported).
 int linear_stream_parts(int rows, int in, int out);
 bool linear_stream_takes(int rows, int in);   // a shadow call with these sizes stays on the streaming kernel
+bool linear_thin_takes(int rows, int in, int64_t out);   // ... with the store epilogue goes to the thin kernel
 // Number of per-row candidate slices the argmax epilogue of a shadow call with these sizes writes (0: unsupported).
 int linear_argmax_parts(int rows, int in, int out);
 // tcgen05 GEMM for many rows (linear_gemm.cu): shadow input only; B200_UNSUPPORTED otherwise.

@@ -655,14 +655,15 @@ __global__ void __launch_bounds__(kThinThreads) linear_thin_kernel(const LinearP
     }
 }
 
+bool linear_thin_takes(int rows, int in, int64_t out) { return (rows >= kGemmRows || in > kMaxIn) && out <= kThinMaxOut && rows <= 512; }
+
 int launch_linear_thin(const LinearParams& p, cudaStream_t stream) {
     const dim3 grid(static_cast<unsigned>(p.rows), static_cast<unsigned>((p.out + kThinFeatures - 1) / kThinFeatures));
     return cuda_status(launch_dependent(linear_thin_kernel, grid, dim3(kThinThreads), 0, stream, p), "linear_thin_kernel launch");
 }
 
 int launch_linear_stream(const LinearParams& p, int epilogue, cudaStream_t stream) {
-    if (p.x_hi && (p.rows >= kGemmRows || p.in > kMaxIn) && epilogue == B200_EPI_STORE && p.out <= kThinMaxOut && p.rows <= 512
-        && p.weight_dtype == B200_BF16 && (p.in & 7) == 0
+    if (p.x_hi && epilogue == B200_EPI_STORE && linear_thin_takes(p.rows, p.in, p.out) && p.weight_dtype == B200_BF16 && (p.in & 7) == 0
         && ((reinterpret_cast<uintptr_t>(p.weight) | reinterpret_cast<uintptr_t>(p.x_hi) | reinterpret_cast<uintptr_t>(p.x_lo)) & 15) == 0)
         return launch_linear_thin(p, stream);
     if (p.x_hi) {

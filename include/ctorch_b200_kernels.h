@@ -146,7 +146,7 @@ typedef struct b200_elementwise_norm {
 
 typedef struct b200_shadow_linear_args {
     const void* x_hi;              /* bf16 [rows, in] */
-    const void* x_lo;              /* may be NULL for calls the dense kernel serves (more than 16 rows or in > 2048): the
+    const void* x_lo;              /* may be NULL for calls of more than 16 rows or with in > 2048: the
                                       activations then count as bf16 - half the operand traffic and tensor-core work */
     int64_t rows, in;
     const void* weight;            /* bf16 [out, in] */
@@ -172,19 +172,20 @@ typedef struct b200_shadow_linear_args {
     int64_t out_stride;            /* SwiGLU epilogue: elements between rows of the output shadow; 0: out/2 (rows follow each other) */
     const struct b200_clamped_unit* unit; /* SwiGLU epilogue: the clamped form of the units; NULL: silu(gate) * up */
 } b200_shadow_linear_args;
-/* Up to 16 rows with in <= 2048: streaming kernel (bulk-TMA weight ring, mma.sync).  More rows or a wider input:
- * dense tcgen05 kernel (TMA operand tiles, accumulator in tensor memory; K split over a thread-block cluster when the
- * tiles are few, a persistent variant for prefill-sized passes), except store-epilogue calls with at most 64 output
- * features (adapter down-projections), which a CUDA-core kernel serves.  B200_UNSUPPORTED when in % 8 != 0. */
+/* Up to 16 rows with in <= 2048, and up to 4 rows of wider inputs: streaming kernel (per-lane cp.async rings of weights, mma.sync).  Otherwise
+ * dense tcgen05 kernels (TMA operand tiles, accumulator in tensor memory): decode batches of up to 256 rows with the weights as the streamed
+ * operand; above, tiles of 128 or 256 features, K split over a thread-block cluster when the tiles are few, persistent variants for
+ * prefill-sized passes.  Store-epilogue calls with at most 64 output features (adapter down-projections) of 17 - 512 rows, or fewer with in >
+ * 2048, are served by a CUDA-core kernel.  B200_UNSUPPORTED when in % 8 != 0. */
 B200_API int b200_linear_shadow(const b200_shadow_linear_args* args, void* stream);
-/* Number of row-sum partials a residual-epilogue call with these sizes writes (its feature tiles), 0 if unsupported. */
+/* Number of row-sum partials a residual-epilogue call with these sizes writes (one per feature tile), 0 if unsupported. */
 B200_API int32_t b200_linear_shadow_parts(int64_t rows, int64_t in, int64_t out);
-/* Number of candidate slices a B200_EPI_ARGMAX call with these sizes writes (one per CTA of the streaming kernel, one per
- * feature tile of the dense kernel), 0 if unsupported. */
+/* Number of candidate slices a B200_EPI_ARGMAX call with these sizes writes (one per warp group of the streaming kernel, up
+ * to two in a CTA; one per feature tile of the dense kernels), 0 if unsupported. */
 B200_API int32_t b200_linear_argmax_parts(int64_t rows, int64_t in, int64_t out);
-/* Name of the kernel family a b200_linear_shadow call with these sizes runs on ("linear_stream_kernel": up to 16 rows;
+/* Name of the kernel family a b200_linear_shadow call with these sizes runs on ("linear_stream_kernel": up to 16 rows, 4 with in > 2048;
  * "linear_decode_kernel": decode batches on tcgen05 with the weights as the streamed operand; "linear_gemm_kernel": more
- * rows; "linear_thin_kernel": at most 64 output features).  For logs and benchmarks. */
+ * rows; "linear_thin_kernel": at most 64 output features, store epilogue).  For logs and benchmarks. */
 B200_API const char* b200_linear_shadow_kernel(int64_t rows, int64_t in, int64_t out);
 /* Launch shape the decode-batch kernel would take for these sizes (host-side; needs no GPU - without one the figures of a
  * 148-SM B200 are used): shape[0..9] = weight tiles per CTA, K split (cluster size), tile groups (grid y), ring stages,

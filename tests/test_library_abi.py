@@ -113,8 +113,8 @@ def test_decoder_options_are_validated_on_the_host():
 
 def test_partial_sum_buffers_follow_the_kernels_tilings():
     """The [parts, rows] buffers that carry per-row sums of squares between kernels are sized from the producers' own
-    tile counts.  With the SwiGLU width below the model width the streaming kernel tiles the down-projection by 8
-    features: d 4096 / hidden 2048 writes 512 partials per row, d 3072 / hidden 2048 writes 384 (host arithmetic only)."""
+    counts: one per 16 features of the streaming kernel, per 128 or 256 of the dense ones; never fewer rows than one
+    per 8 features, which callers may have laid buffers out for (host arithmetic only)."""
     l = B.lib()
     assert l.dl_b200_shadow_partial_rows(4096, 2048) >= 512
     assert l.dl_b200_shadow_partial_rows(3072, 2048) >= 384
@@ -126,13 +126,15 @@ def test_partial_sum_buffers_follow_the_kernels_tilings():
 
 def test_shadow_linear_dispatch_by_row_count():
     """Which kernel family serves a shadow linear: the streaming kernel up to 16 rows (inner size up to 2048), the
-    decode-batch kernel up to 256 rows, the prefill kernel above, the thin kernel for adapter down-projections."""
+    decode-batch kernel up to 256 rows, the prefill kernels above, the thin kernel for adapter down-projections."""
     name = lambda rows, inner, out: B.lib().b200_linear_shadow_kernel(rows, inner, out).decode()
     assert name(1, 768, 2304) == name(16, 2048, 32000) == "linear_stream_kernel"
     assert name(8, 4096, 6144) == "linear_decode_kernel"          # few rows, but wider than the streaming kernel's ring
     assert name(17, 768, 2304) == name(128, 2048, 16384) == name(256, 8192, 2048) == "linear_decode_kernel"
     assert name(257, 2048, 16384) == name(8192, 2048, 3072) == "linear_gemm_kernel"
-    assert name(32, 4096, 32) == "linear_thin_kernel"
+    assert name(4, 4096, 6144) == "linear_stream_kernel" and name(5, 4096, 6144) == "linear_decode_kernel"   # wide inputs: up to 4 rows
+    assert name(32, 4096, 32) == name(3, 4096, 64) == name(512, 768, 64) == "linear_thin_kernel"
+    assert name(513, 768, 64) == "linear_gemm_kernel" and name(16, 2048, 64) == "linear_stream_kernel"
 
 
 def test_tiles_of_long_passes_follow_the_epilogue():
