@@ -197,7 +197,8 @@ __device__ __forceinline__ Span<V> turned_span(const ChunkParams& p, const float
 }
 
 // Bound by its chain of loads (the row's place, its values, angles and weights), so by the CTAs that an SM holds: five, at 48 registers (8192 rows of
-// 16 / 4 heads of 64: 77 us with four at 64, 68 so; six and more spill).
+// 16 / 4 heads of 64: 77 us with four at 64, 68 so; 4096 rows by norm kind, bf16 cache: 33 -> 29, 25 -> 21 and 35 -> 32 us although up to five values of
+// a thread go to the stack; with six CTAs many do).
 constexpr int kPrepareThreads = 256, kUnitSlice = 1024;
 // grid (rows, 1 + slices of the units)
 

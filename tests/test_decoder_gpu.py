@@ -310,7 +310,13 @@ def test_config2_width_short_context_bf16():
     out = np.empty(spec["batch"], dtype=np.int64)
     for step in range(1, spec["steps"]):
         gen.step_host(np.ascontiguousarray(want_tokens[:, step - 1]), out)
-        assert rel(gen.logits(), want_logits[step]) < BF16_TOL, step
+        got, want = gen.logits(), want_logits[step]
+        assert rel(got, want) < BF16_TOL, step
+        # the choice is the oracle's wherever its two leading logits lie farther apart than this row's logits are off, and always the row's own
+        lead = np.partition(want.astype(np.float64), -2, axis=-1)[:, -2:]
+        clear = lead[:, 1] - lead[:, 0] > 2 * np.abs(got.astype(np.float64) - want).max(axis=-1)
+        assert clear.any() and np.array_equal(out[clear], want.argmax(axis=-1)[clear])
+        assert np.array_equal(out, got.argmax(axis=-1))
     # f32 cache switch: the only remaining deviation is summation order
     exact = B.DecoderModel(spec, weights, cache_dtype="f32")
     port.new_cache()

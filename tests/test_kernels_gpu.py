@@ -638,6 +638,61 @@ def test_wide_linear_tiles(rows, inner, out, epilogue):
     test_dense_tensor_core_linear(rows, inner, out, epilogue)
 
 
+@pytest.mark.parametrize("rows,inner,out,planes", [(1030, 136, 2568, 1), (1030, 136, 2568, 2), (2, 2056, 1000, 1), (2, 2056, 1000, 2), (9, 264, 1002, 2)])
+@pytest.mark.parametrize("norm", ["bf16", "f32", "tanh"])
+def test_residual_epilogues_fold_the_next_norm(rows, inner, out, planes, norm):
+    """The residual epilogue's output planes hold the rows times the next norm's weight, or behind Dynamic Tanh: the register epilogue of long
+    passes and the streaming kernels', with one and with two planes of input.  Planes hold 16 bits: 2^-16 beside the f32 sums' 2e-5."""
+    l = B.lib()
+    g = torch.Generator(device="cuda").manual_seed(rows + out)
+    normal = lambda *shape: torch.randn(shape, generator=g, device="cuda")
+    x, residual, w = normal(rows, inner), normal(rows, out), (normal(out, inner) * inner ** -0.5).bfloat16()
+    hi = x.bfloat16()
+    lo = (x - hi.float()).bfloat16()
+    weight, bias = 1 + 0.1 * normal(out), 0.1 * normal(out)
+    if norm == "bf16":
+        weight = weight.bfloat16()
+    y = torch.full((rows, out), float("nan"), device="cuda")
+    got = [torch.full((rows, out), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    squares = torch.full((l.b200_linear_shadow_parts(rows, inner, out), rows), float("nan"), device="cuda")
+    args = B.ShadowLinearArgs(x_hi=hi.data_ptr(), x_lo=lo.data_ptr() if planes == 2 else None, rows=rows, inner=inner, weight=w.data_ptr(), out=out, epilogue=1,
+                              residual=residual.data_ptr(), y=y.data_ptr(), out_hi=got[0].data_ptr(), out_lo=got[1].data_ptr())
+    tanh = B.ElementwiseNorm(0.7, weight.data_ptr(), bias.data_ptr())
+    if norm == "tanh":
+        args.out_norm = C.pointer(tanh)
+    else:
+        args.out_norm_weight, args.out_norm_dtype, args.sumsq_out = weight.data_ptr(), B.BF16 if norm == "bf16" else B.F32, squares.data_ptr()
+    torch.cuda.synchronize()
+    B.kcheck(l.b200_linear_shadow(C.byref(args), stream()))
+    sync()
+    want = residual.double() + (hi.double() + (lo.double() if planes == 2 else 0)) @ w.double().T
+    normed = torch.tanh(0.7 * want) * weight.double() + bias.double() if norm == "tanh" else want * weight.double()
+    off = lambda a, b: float((a.double() - b).norm() / b.norm())
+    assert off(y, want) < 2e-5 and off(got[0].double() + got[1].double(), normed) < 4e-5
+    if norm != "tanh":
+        assert off(squares.sum(0), want.square().sum(1)) < 2e-5
+
+
+@pytest.mark.parametrize("hd,heads,kv_heads,n,prefix,L", [(64, 12, 4, 10, 70, 41), (128, 8, 2, 30, 100, 17), (64, 8, 2, 3, 1100, 1), (128, 8, 2, 3, 2500, 1)])
+def test_attention_planes_hold_the_f32_result(hd, heads, kv_heads, n, prefix, L):
+    """Prefill blocks and splits merged inside a cluster, written as planes: the f32 result and what its bf16 rounding leaves."""
+    rng = np.random.default_rng(hd + n)
+    cap = prefix + L
+    cache = Cache(B.BF16, n, kv_heads, hd, cap)
+    cache.append(*(rng.standard_normal((n, kv_heads, cap, hd), dtype=np.float32) for _ in range(2)))
+    cache.set_lengths(np.full(n, prefix, dtype=np.int32))
+    q = rng.standard_normal((n * L, heads, hd), dtype=np.float32)
+    plain = torch.from_numpy(attention(q, cache, L, heads, cap)).cuda()
+    qd = dev(q)
+    hi, lo = (torch.zeros((n * L, heads * hd), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    need = B.lib().b200_attention_scratch_bytes(n * L, heads, kv_heads, hd, cap, 64)
+    scratch = torch.empty((need,), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    B.kcheck(B.lib().b200_attention_decode_shadow(qd.data_ptr(), n * L, L, heads, cache.h, cap, 1, scratch.data_ptr(), need, hi.data_ptr(), lo.data_ptr(), stream()))
+    sync()
+    assert torch.equal(hi, plain.bfloat16()) and torch.equal(lo, (plain - hi.float()).bfloat16())
+
+
 @pytest.mark.parametrize("cache_dtype,heads,kv_heads,hd", [(B.BF16, 16, 4, 64), (B.F32, 24, 24, 32)])
 def test_wide_linear_appends_q_k_v(cache_dtype, heads, kv_heads, hd):
     """The q|k|v epilogue of a long pass: rotation, queries, cache entries on shuffled pages, behind cached tokens."""
@@ -899,10 +954,12 @@ def test_peer_memory_sum_gives_up_when_a_rank_never_arrives():
     assert float(x.sum()) == 8.0
 
 
-@pytest.mark.parametrize("rows,inner,out", [(40, 768, 1280), (256, 2048, 3072), (32, 4096, 1024)])
+@pytest.mark.parametrize("rows,inner,out", [(40, 768, 1280), (256, 2048, 3072), (32, 4096, 1024), (4, 2056, 1000), (3, 4096, 128), (5, 4096, 128),
+                                            (1030, 128, 2568)])
 def test_dense_linear_with_single_plane_activations(rows, inner, out):
-    """x_lo = NULL: the dense kernel multiplies the hi plane only, i.e. activations rounded to bf16.  The result must equal
-    the oracle's linear of the ROUNDED activations to f32 accuracy, and the unrounded one within bf16 resolution."""
+    """x_lo = NULL: the kernels multiply the hi plane only, i.e. activations rounded to bf16 (also the streaming kernel, for wide inputs of at
+    most 4 rows, and the tiles of 256 features).  The result must equal the oracle's linear of the ROUNDED activations to f32 accuracy,
+    and the unrounded one within bf16 resolution."""
     l = B.lib()
     rng = np.random.default_rng(rows + out)
     x = rng.standard_normal((rows, inner), dtype=np.float32)
@@ -955,11 +1012,13 @@ def test_tensordot_matches_the_reference_rule(a_shape, b_shape, axes_a, axes_b):
     assert b"must be distinct" in B.lib().dl_last_error()
 
 
-@pytest.mark.parametrize("rows,inner,out,epilogue", [(4, 512, 1024, 1), (40, 1024, 512, 1), (200, 768, 1280, 0), (16, 2048, 768, 0)])
+@pytest.mark.parametrize("rows,inner,out,epilogue", [(4, 512, 1024, 1), (40, 1024, 512, 1), (200, 768, 1280, 0), (16, 2048, 768, 0), (300, 128, 640, 1),
+                                                     (1030, 128, 2568, 0), (1024, 128, 2560, 1)])
 def test_projection_pushes_its_rows_to_extra_destinations(rows, inner, out, epilogue):
     """y_copies of a shadow linear: every extra destination receives exactly the rows written to y - the mechanism by which
     a tensor-parallel rank's projection deposits its partial sums in the peers' memory from its own epilogue (here the
-    destinations are buffers of the same GPU).  Streaming kernel (4 and 16 rows), decode-batch kernel (40), prefill kernel (200)."""
+    destinations are buffers of the same GPU).  Streaming kernel (4 and 16 rows), decode-batch kernel (40, 200), prefill kernels (300; 1030, 1024: tiles
+    of 256 features)."""
     l = B.lib()
     rng = np.random.default_rng(rows + out)
     x = rng.standard_normal((rows, inner), dtype=np.float32)
